@@ -338,16 +338,100 @@ int grant_shared_memory(const mpcf_solver* s)
     return MPCF_OK;
 }
 
-int persistent_grid(mpcf_solver* s, int ty)
+// Resident CTAs per SM of the stage kernel at tile height ty.
+int resident_ctas(const mpcf_solver* s, int ty, bool persist, bool tma)
 {
-    StageKernelInfo I = stage_info(s, ty, true, false, s->tma != 0);
+    const StageKernelInfo I = stage_info(s, ty, persist, false, tma);
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, I.fn, stage_block_threads(ty), I.smem) != cudaSuccess || nb < 1)
+    if (!I.fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, I.fn, stage_block_threads(ty), I.smem) != cudaSuccess || nb < 1)
     {
         cudaGetLastError();
         nb = 1;
     }
-    return std::min(s->ntiles, nb * s->num_sms);
+    return nb;
+}
+
+// Chunk depth with the shortest expected stage for tiles of height ty, from
+// how a stage's time was measured to depend on it (B200, 32 x 8 tiles): a CTA
+// takes its depth plus a start-up of about one slab (12.4 us at depth 1, 3.85
+// us per further slab in the mixed form; 27 and 14.4 in FP32 reference
+// rounding), an SM with two CTAs gives each 0.66 (fast FP32 forms) or 0.78
+// (reference rounding) of the speed it has alone, and CTAs beyond the
+// resident ones wait for a slot.  So the best depth is the one whose CTAs
+// fill whole rounds of resident slots with the least start-up: 64^3 takes 4
+// (35 us per stage in the mixed form; 16 gives 70, 2 gives 40), 192^3 48 to
+// 64, 256^3 32 to 64.  Domains of different sizes (several per launch) fill
+// the slots like a list schedule: total work plus half a CTA's length.
+// `nd` leading domains share a launch.
+int best_depth(const mpcf_solver* s, int ty, int nd, int nb, double* cost_out = nullptr)
+{
+    const double start = 1.0, alone = s->pol == MPCF_PREC_FP32 || s->pol == MPCF_PREC_MIXED ? 0.66 : 0.78;
+    const long long sms = s->num_sms, slots = sms * nb;
+    int deepest = 0;
+    bool even = true;
+    for (int d = 0; d < nd; ++d)
+    {
+        const DomDev& D = s->hdoms[d];
+        deepest = std::max(deepest, D.nz);
+        even = even && D.nx == s->hdoms[0].nx && D.ny == s->hdoms[0].ny && D.nz == s->hdoms[0].nz;
+    }
+    int best = deepest, last = 0;
+    double best_cost = 1e300;
+    for (int n = 1; n <= std::min(deepest, 512); ++n)
+    {
+        const int dz = (deepest + n - 1) / n;
+        if (dz == last) continue;
+        last = dz;
+        long long ctas = 0;
+        double work = 0;
+        for (int d = 0; d < nd; ++d)
+        {
+            const DomDev& D = s->hdoms[d];
+            const long long txy = (long long)((D.nx + 31) / 32) * ((D.ny + ty - 1) / ty), cz = (D.nz + dz - 1) / dz;
+            ctas += txy * cz;
+            work += (double)txy * (D.nz + start * cz);
+        }
+        double cost;
+        if (even)
+        {
+            const long long rem = ctas % slots;
+            const double tail = rem == 0 ? 0.0 : (nb > 1 && rem <= sms ? alone : 1.0);
+            cost = ((double)(ctas / slots) + tail) * (work / ctas);
+        }
+        else cost = work / slots + 0.5 * (dz + start);
+        cost = std::max(cost, (nb > 1 && ctas <= sms ? alone : 1.0) * (dz + start));
+        if (cost < best_cost * 0.995) { best_cost = cost; best = dz; }
+    }
+    if (cost_out) *cost_out = best_cost;
+    return best;
+}
+
+// The tiling a new solver starts with, for launches over its first `nd`
+// domains: 32 x 8 columns (the fastest height of every form at 64^3 to 512^3:
+// mixed 256^3 3.9 ms a step against 4.5 at height 7 and 5.6 at 3), bulk
+// copies, the depth above; the fast FP32 forms schedule more CTAs than
+// resident slots through persistent ones (256^3: 1.23 against 1.29 ms a
+// stage; the other forms gain nothing and skip the counter's reset).
+void default_tiling(mpcf_solver* s, int nd)
+{
+    bool tma = false;
+    for (int d = 0; d < nd; ++d) tma = tma || ((size_t)s->hdoms[d].nx * s->esz) % 16 == 0;
+    s->ty = 8;
+    s->tma = 1;                       // dropped by apply_tiling when no domain qualifies
+    const int nb = resident_ctas(s, s->ty, false, tma);
+    s->dz = best_depth(s, s->ty, nd, nb);
+    long long ctas = 0;
+    for (int d = 0; d < nd; ++d)
+    {
+        const DomDev& D = s->hdoms[d];
+        ctas += (long long)((D.nx + 31) / 32) * ((D.ny + s->ty - 1) / s->ty) * ((D.nz + s->dz - 1) / s->dz);
+    }
+    s->persist = (s->pol == MPCF_PREC_FP32 || s->pol == MPCF_PREC_MIXED) && ctas > (long long)nb * s->num_sms;
+}
+
+int persistent_grid(mpcf_solver* s, int ty)
+{
+    return std::min(s->ntiles, resident_ctas(s, ty, true, s->tma != 0) * s->num_sms);
 }
 
 StageArgs stage_args(mpcf_solver* s, double a, double b, bool sums)
@@ -593,10 +677,7 @@ int mpcf_create(mpcf_solver** out, int ndomains, const int* dims, const int* bc,
     { cudaGetLastError(); return bail(fail(MPCF_ERR_NOMEM, "cudaMallocHost failed")); }
 
     if ((rc = grant_shared_memory(s))) return bail(rc);
-    s->ty = 7;
-    s->dz = 64;
-    s->persist = 0;
-    s->tma = 1;                       // dropped by apply_tiling when no domain qualifies
+    default_tiling(s, ndomains);
     if ((rc = apply_tiling(s))) return bail(rc);
     *out = s;
     return MPCF_OK;
@@ -1249,13 +1330,8 @@ int mpcf_create_window(mpcf_solver** out, int nx, int ny, int nz, int nslices, i
         D.gdim[0] = nx; D.gdim[1] = ny; D.gdim[2] = nz;
     }
     DeviceGuard g(s->device);
-    if (cudaMemcpyAsync(s->ddoms, s->hdoms.data(), sizeof(DomDev) * s->ndom, cudaMemcpyHostToDevice, s->stream) != cudaSuccess ||
-        cudaStreamSynchronize(s->stream) != cudaSuccess)
-    {
-        cudaGetLastError();
-        mpcf_destroy(s);
-        return fail(MPCF_ERR_CUDA, "window set-up copy failed");
-    }
+    default_tiling(s, 1);             // a stage launch covers one slot
+    if ((rc = apply_tiling(s))) { mpcf_destroy(s); return rc; }
     *out = s;
     return MPCF_OK;
 }
@@ -2256,12 +2332,11 @@ int mpcf_time_stages(mpcf_solver* s, int reps, double dtinvh, double* ms_per_sta
 }
 
 // z-chunk depths the autotuner tries for tile height ty: 16, 32, 64 and 128
-// below the deepest domain, and the whole depth.  When 16-deep chunks do not
-// fill one wave of resident CTAs (small domains), also the shallowest depth
-// whose CTAs still fit in one wave, and 8: a CTA walks its chunk slab by
-// slab, so there the chunk depth is the latency of the stage (64^3, mixed:
-// 4-deep chunks of 32x8 tiles, 256 CTAs, run a step 1.9x faster than the
-// best 16-deep tiling).
+// below the deepest domain, the whole depth, and the depth the model of
+// best_depth picks.  When 16-deep chunks do not fill one wave of resident
+// CTAs (small domains), also the shallowest depth whose CTAs still fit in
+// one wave, and 8: a CTA walks its chunk slab by slab, so there the chunk
+// depth is the latency of the stage.
 static std::vector<int> dz_candidates(mpcf_solver* s, int ty, int maxn, bool tma)
 {
     auto tiles = [&](int dz)
@@ -2273,13 +2348,8 @@ static std::vector<int> dz_candidates(mpcf_solver* s, int ty, int maxn, bool tma
     std::vector<int> dzs;
     for (int v : {16, 32, 64, 128}) if (v < maxn) dzs.push_back(v);
     dzs.push_back(maxn);
-    const StageKernelInfo I = stage_info(s, ty, false, false, tma);
-    int nb = 0;
-    if (!I.fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, I.fn, stage_block_threads(ty), I.smem) != cudaSuccess || nb < 1)
-    {
-        cudaGetLastError();
-        nb = 1;
-    }
+    const int nb = resident_ctas(s, ty, false, tma);
+    dzs.push_back(best_depth(s, ty, s->ndom, nb));
     const long long slots = (long long)nb * s->num_sms;
     if (maxn > 4 && tiles(std::min(16, maxn)) < slots)
     {
@@ -2329,6 +2399,11 @@ int mpcf_autotune(mpcf_solver* s, int reps, int* best3, double* best_ms)
         for (int i = 0; i < 4 && !rc; ++i)
         {
             if (!valid_ty(s, tys[i])) continue;
+            // 8 rows are the fastest height; another is tried where its tiles
+            // cover a domain's rows with fewer rows in all
+            bool fewer = tys[i] == 8;
+            for (auto& D : s->hdoms) fewer = fewer || (D.ny + tys[i] - 1) / tys[i] * tys[i] < (D.ny + 7) / 8 * 8;
+            if (!fewer) continue;
             for (int dz : dz_candidates(s, tys[i], maxn, can_tma))
             {
                 for (int f = 0; f < 4 && !rc; ++f)
