@@ -110,7 +110,7 @@ struct mpcf_solver
     int bubbles_cap = 0;
     void* host_stage = nullptr;     // pinned host scratch (ndom doubles/elems)
 
-    void* tmaps = nullptr;          // ndom * 4 CUtensorMap (128 B each)
+    void* tmaps = nullptr;          // ndom * 5 CUtensorMap (128 B each)
 
     // linked z-slabs (lower, upper) and their device copy
     std::vector<int> links;         // 2 per link
@@ -153,12 +153,9 @@ struct mpcf_solver
 
 namespace {
 
-// Tile heights with stage-kernel instances: 3 and 7 rows (CTAs of 4 and 8
-// warps: one warp per row plus the helper warp), 8 rows (8 warps, no
-// helper), and 15 rows (16 warps) for the FP32 reference-rounding form.
-// Threads of one stage CTA: a warp per row, plus the helper warp for
-// heights 2^n - 1 (TileShape in mpcf_stage.cuh).
-int stage_block_threads(int ty) { return ((ty + 1) & ty) == 0 ? 32 * (ty + 1) : 32 * ty; }
+// Tile heights with stage-kernel instances: 3, 7 and 8 rows, and 15 for the
+// FP32 reference-rounding form.  Threads of one stage CTA: a warp per row.
+int stage_block_threads(int ty) { return 32 * ty; }
 
 bool valid_ty(const mpcf_solver* s, int ty)
 {
@@ -216,7 +213,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
 
 // Tensor maps of every domain for the current tile height: per state buffer a
 // 40 x (ty+6) x 1 x 7 halo box and a 32 x ty x 1 x 7 interior box over the
-// 4-D view (x, y, z, field) of the buffer.  A domain qualifies when its row
+// 4-D view (x, y, z, field) of the buffer, and the interior box of the register.  A domain qualifies when its row
 // and plane pitches are multiples of 16 bytes (nx*elem % 16 == 0).
 bool any_tma_ok(const mpcf_solver* s)
 {
@@ -226,7 +223,7 @@ bool any_tma_ok(const mpcf_solver* s)
 
 int encode_tensor_maps(mpcf_solver* s)
 {
-    std::vector<CUtensorMap> h((size_t)s->ndom * 4);
+    std::vector<CUtensorMap> h((size_t)s->ndom * 5);
     memset(h.data(), 0, h.size() * sizeof(CUtensorMap));
     PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
     for (int d = 0; d < s->ndom; ++d)
@@ -235,22 +232,24 @@ int encode_tensor_maps(mpcf_solver* s)
         const size_t e = s->esz;
         bool ok = enc != nullptr && ((size_t)D.nx * e) % 16 == 0 && ((size_t)D.nx * D.ny * e) % 16 == 0 &&
                   ((size_t)D.fs * e) % 16 == 0;
-        for (int b = 0; b < 2 && ok; ++b)
-            for (int box = 0; box < 2 && ok; ++box)
-            {
-                // over the stored planes, ghost planes included (the kernel
-                // adds zlo to its z coordinates)
-                const cuuint64_t dims[4] = {(cuuint64_t)D.nx, (cuuint64_t)D.ny, (cuuint64_t)(D.nz + D.zlo + D.zhi), 7};
-                const cuuint64_t strides[3] = {(cuuint64_t)D.nx * e, (cuuint64_t)D.nx * D.ny * e, (cuuint64_t)D.fs * e};
-                const cuuint32_t boxd[4] = {box == 0 ? 40u : 32u, (cuuint32_t)(box == 0 ? s->ty + 6 : s->ty), 1u, 7u};
-                const cuuint32_t estr[4] = {1, 1, 1, 1};
-                CUresult r = enc(&h[(size_t)d * 4 + b * 2 + box],
-                                 e == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
-                                 4, (char*)D.U[b] - (size_t)D.zlo * D.nx * D.ny * e, dims, strides, boxd, estr,
-                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-                ok = (r == CUDA_SUCCESS);
-            }
+        // buffer 0, buffer 1: halo box and interior box over the stored
+        // planes, ghost planes included (the kernel adds zlo to its z
+        // coordinates); register: interior box over the domain's own planes
+        for (int i = 0; i < 5 && ok; ++i)
+        {
+            const bool reg = i == 4, halo = !reg && (i & 1) == 0;
+            const size_t zlo = reg ? 0 : D.zlo;
+            const cuuint64_t dims[4] = {(cuuint64_t)D.nx, (cuuint64_t)D.ny, (cuuint64_t)(reg ? D.nz : D.nz + D.zlo + D.zhi), 7};
+            const cuuint64_t strides[3] = {(cuuint64_t)D.nx * e, (cuuint64_t)D.nx * D.ny * e, (cuuint64_t)D.fs * e};
+            const cuuint32_t boxd[4] = {halo ? 40u : 32u, (cuuint32_t)(halo ? s->ty + 6 : s->ty), 1u, 7u};
+            const cuuint32_t estr[4] = {1, 1, 1, 1};
+            CUresult r = enc(&h[(size_t)d * 5 + i],
+                             e == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+                             4, (char*)(reg ? D.R : D.U[i >> 1]) - zlo * D.nx * D.ny * e, dims, strides, boxd, estr,
+                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+            ok = (r == CUDA_SUCCESS);
+        }
         D.tma_ok = ok ? 1 : 0;
     }
     CK(cudaMemcpyAsync(s->tmaps, h.data(), h.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, s->stream));
@@ -590,7 +589,10 @@ int mpcf_elem_size(int precision)
     return (precision == MPCF_PREC_FP64 || precision == MPCF_PREC_FP64_FAST) ? 8 : 4;
 }
 
-int mpcf_create(mpcf_solver** out, int ndomains, const int* dims, const int* bc, int precision, int device)
+// mpcf_create; per_launch: how many leading domains a stage launch covers
+// (all, or one slot of a windowed solver), which sizes the default tiling.
+static int create_solver(mpcf_solver** out, int ndomains, const int* dims, const int* bc, int precision, int device,
+                         int per_launch)
 {
     if (!out) return fail(MPCF_ERR_ARG, "null output handle");
     *out = nullptr;
@@ -665,7 +667,7 @@ int mpcf_create(mpcf_solver** out, int ndomains, const int* dims, const int* bc,
     if ((rc = dev_alloc(s, (void**)&s->sums, 8 * 5 * ndomains))) return bail(rc);
     if ((rc = dev_alloc(s, (void**)&s->err, 16))) return bail(rc);
     if ((rc = dev_alloc(s, (void**)&s->counter, 16))) return bail(rc);
-    if ((rc = dev_alloc(s, &s->tmaps, (size_t)128 * 4 * ndomains))) return bail(rc);
+    if ((rc = dev_alloc(s, &s->tmaps, (size_t)128 * 5 * ndomains))) return bail(rc);
     cudaMemsetAsync(s->sos_bits, 0, 8 * ndomains, s->stream);
     cudaMemsetAsync(s->dtinvh, 0, 8 * ndomains, s->stream);
     cudaMemsetAsync(s->dt, 0, 8 * ndomains, s->stream);
@@ -677,10 +679,15 @@ int mpcf_create(mpcf_solver** out, int ndomains, const int* dims, const int* bc,
     { cudaGetLastError(); return bail(fail(MPCF_ERR_NOMEM, "cudaMallocHost failed")); }
 
     if ((rc = grant_shared_memory(s))) return bail(rc);
-    default_tiling(s, ndomains);
+    default_tiling(s, per_launch);
     if ((rc = apply_tiling(s))) return bail(rc);
     *out = s;
     return MPCF_OK;
+}
+
+int mpcf_create(mpcf_solver** out, int ndomains, const int* dims, const int* bc, int precision, int device)
+{
+    return create_solver(out, ndomains, dims, bc, precision, device, ndomains);
 }
 
 int mpcf_destroy(mpcf_solver* s)
@@ -1313,7 +1320,7 @@ int mpcf_create_window(mpcf_solver** out, int nx, int ny, int nz, int nslices, i
         bcs[6 * d + 4] = bcs[6 * d + 5] = MPCF_BC_HALO;
     }
     mpcf_solver* s = nullptr;
-    int rc = mpcf_create(&s, ns, dims.data(), bcs.data(), precision, device);
+    int rc = create_solver(&s, ns, dims.data(), bcs.data(), precision, device, 1);
     if (rc) return rc;
     s->win_nz = nz;
     s->win_nslices = nslices;
@@ -1330,8 +1337,13 @@ int mpcf_create_window(mpcf_solver** out, int nx, int ny, int nz, int nslices, i
         D.gdim[0] = nx; D.gdim[1] = ny; D.gdim[2] = nz;
     }
     DeviceGuard g(s->device);
-    default_tiling(s, 1);             // a stage launch covers one slot
-    if ((rc = apply_tiling(s))) { mpcf_destroy(s); return rc; }
+    if (cudaMemcpyAsync(s->ddoms, s->hdoms.data(), sizeof(DomDev) * s->ndom, cudaMemcpyHostToDevice, s->stream) != cudaSuccess ||
+        cudaStreamSynchronize(s->stream) != cudaSuccess)
+    {
+        cudaGetLastError();
+        mpcf_destroy(s);
+        return fail(MPCF_ERR_CUDA, "window set-up copy failed");
+    }
     *out = s;
     return MPCF_OK;
 }

@@ -29,8 +29,8 @@
 //
 // Primitive index convention used throughout the device code:
 //   0 rho, 1 u, 2 v, 3 w, 4 p, 5 G = 1/(gamma-1), 6 P = gamma*pc/(gamma-1)
-// Face output slots: 0..6 fluxes of (rho, rho u, rho v, rho w, E, G, P),
-//   7 Gm, 8 Gp, 9 Pm, 10 Pp, 11 u* (extra-term velocity).
+// Face outputs: 0..6 fluxes of (rho, rho u, rho v, rho w, E, G, P),
+//   7 u* (extra-term velocity).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -113,6 +113,30 @@ template <class T> __device__ __forceinline__ T beta_g(const T x, const T y, con
     return x*(x*(T)(10./3.) - y*(T)(31./3.) + z*(T)(11./3.)) + y*(y*(T)(25./3.) - z*(T)(19./3.)) + z*z*(T)(4./3.);
 }
 
+// Correctly rounded reciprocal without a branch, for arguments whose
+// reciprocal is far from under- and overflow: Newton-Raphson from the
+// special-function unit's approximation, the last step on the exact residual
+// 1 - x y of an approximation y within one unit in the last place, which
+// rounds correctly unless x's mantissa is all ones (Markstein, "Computation
+// of elementary functions on the IBM RISC System/6000 processor", 1990).  Other
+// arguments (0, subnormal, huge, infinite, NaN) give a NaN or a wrong value:
+// the caller checks.
+__device__ __forceinline__ double rcp_rn(const double x)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = __fma_rn(-x, y, 1.0);
+    y = __fma_rn(y, __fma_rn(e, e, e), y);      // y (1 + e + e^2): 3 times the correct bits
+    return __fma_rn(y, __fma_rn(-x, y, 1.0), y);
+}
+
+// Whether a positive x (or a NaN, which is not) lies in [lo, hi), powers of
+// two: an integer comparison of the exponents, off the FP64 pipe.
+__device__ __forceinline__ bool in_range(const double x, const double lo, const double hi)
+{
+    return (unsigned)(__double2hiint(x) - __double2hiint(lo)) < (unsigned)(__double2hiint(hi) - __double2hiint(lo));
+}
+
 // Both edge values of one cell in the reference-rounding policies, from the
 // cells y0..y4 = l-2..l+2 (GPUonly.cuh:99-194):
 //   R, the minus side of face l+1/2: indicators (is0, is1, is2) =
@@ -129,8 +153,14 @@ template <class T> __device__ __forceinline__ T beta_g(const T x, const T y, con
 // edges of a cell are the same operations on the same values, so they are
 // evaluated once here.  Every other operation is the reference's in its
 // order, so R and L are bit-identical to its per-face results.
-template <class Pol>
-__device__ __forceinline__ void weno_cell_ref(const typename Pol::T y0, const typename Pol::T y1,
+//
+// kBranchFree: the reciprocals through rcp_rn; returns whether both sums of
+// weights lie where those are exact (false also when a sum is NaN, which a
+// zero or infinite pf, ph or pg leads to).  The compiler's own division
+// carries a branch to its slow path for each of the five reciprocals, which
+// cuts the code of a cell's 7 quantities into pieces too short to overlap.
+template <class Pol, bool kBranchFree>
+__device__ __forceinline__ bool weno_cell_ref(const typename Pol::T y0, const typename Pol::T y1,
         const typename Pol::T y2, const typename Pol::T y3, const typename Pol::T y4,
         typename Pol::T& R, typename Pol::T& L)
 {
@@ -140,16 +170,23 @@ __device__ __forceinline__ void weno_cell_ref(const typename Pol::T y0, const ty
     const T ph = beta_h<T>(y1, y2, y3) + (T)MPCF_WENOEPS;
     const T pg = beta_g<T>(y2, y3, y4) + (T)MPCF_WENOEPS;
     // the 10.0 literal promotes these to double (GPUonly.cuh:111-113)
-    const double qf = ((T)1)/(10.0*pf*pf);
-    const double qh = ((T)1)/(10.0*ph*ph);
-    const double qg = ((T)1)/(10.0*pg*pg);
+    const double xf = 10.0*pf*pf, xh = 10.0*ph*ph, xg = 10.0*pg*pg;
+    const double qf = kBranchFree ? rcp_rn(xf) : ((T)1)/xf;
+    const double qh = kBranchFree ? rcp_rn(xh) : ((T)1)/xh;
+    const double qg = kBranchFree ? rcp_rn(xg) : ((T)1)/xg;
     const T a1 = (T)((T)(6)*qh);
     const T lo = dmin(dmin(y1, y2), y3);
     const T hi = dmax(dmax(y1, y2), y3);
+    bool exact = true;
+    static_assert(!kBranchFree || sizeof(T) == 8, "branch-free: FP64 only");
+    const double kLo = 0x1p-900, kHi = 0x1p900;
     {
         // minus side: indicators (f, h, g)
         const T a0 = (T)((T)(1)*qf), a2 = (T)((T)(3)*qg);
-        const T inv = ((T)1)/(a0 + a1 + a2);
+        const T sum = a0 + a1 + a2;
+        T inv;
+        if constexpr (kBranchFree) { exact = sum >= kLo && sum <= kHi; inv = rcp_rn(sum); }
+        else                       inv = ((T)1)/sum;
         const T w0 = a0 * inv, w1 = a1 * inv, w2 = 1 - w0 - w1;
         const T r = w0*((T)(1.0/3.)*y0-(T)(7./6.)*y1+(T)(11./6.)*y2) + w1*(-(T)(1./6.)*y1+(T)(5./6.)*y2+(T)(1./3.)*y3) + w2*((T)(1./3.)*y2+(T)(5./6.)*y3-(T)(1./6.)*y4);
         R = dmin(dmax(r, lo), hi);
@@ -157,42 +194,61 @@ __device__ __forceinline__ void weno_cell_ref(const typename Pol::T y0, const ty
     {
         // plus side: indicators (g, h, f)
         const T a0 = (T)((T)(1)*qg), a2 = (T)((T)(3)*qf);
-        const T inv = ((T)1)/(a0 + a1 + a2);
+        const T sum = a0 + a1 + a2;
+        T inv;
+        if constexpr (kBranchFree) { exact = exact && sum >= kLo && sum <= kHi; inv = rcp_rn(sum); }
+        else                       inv = ((T)1)/sum;
         const T w0 = a0 * inv, w1 = a1 * inv, w2 = 1 - w0 - w1;
         const T r = w0*((T)(1./3.)*y4-(T)(7./6.)*y3+(T)(11./6.)*y2) + w1*(-(T)(1./6.)*y3+(T)(5./6.)*y2+(T)(1./3.)*y1) + w2*((T)(1./3.)*y2+(T)(5./6.)*y1-(T)(1./6.)*y0);
         L = dmin(dmax(r, lo), hi);
     }
+    return exact;
 }
 
 // ---------------------------------------------------------------------------
-// Packed single-precision pairs.  sm_100 executes fma / add / mul on two
-// FP32 lanes in one instruction (round-to-nearest per lane, the same result
-// as two scalar instructions).  The face pipeline is bound by instruction
-// issue, so every left/right-symmetric computation runs as one pair.
+// Explicitly rounded operations on one value (float, double) or on a pair of
+// floats.  sm_100 executes fma / add / mul on two FP32 lanes in one
+// instruction, each lane rounded like the scalar instruction; the face
+// pipeline is bound by instruction issue, so the fast FP32 forms reconstruct
+// two quantities at a time.  No operation here may be contracted with
+// another, and no sum below takes a product that a code generator could fuse:
+// an edge value is the same bits whether a pair, a single value, an interior
+// cell or a ghost cell produced it.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float2 f2(const float a, const float b) { return make_float2(a, b); }
-__device__ __forceinline__ float2 f2s(const float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 add2(const float2 a, const float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 sub2(const float2 a, const float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
-__device__ __forceinline__ float2 mul2(const float2 a, const float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 fma2(const float2 a, const float2 b, const float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 rcp2(const float2 a) { return make_float2(rcp_approx(a.x), rcp_approx(a.y)); }
-// HLLC upwind blend w.x * F.x + w.y * F.y of a (left, right) flux pair
-__device__ __forceinline__ float blend2(const float2 w, const float2 F) { const float2 t = mul2(F, w); return t.x + t.y; }
-// The same pair operations in double precision (the fast FP64 form), lane
-// by lane: there are no packed FP64 instructions.
-__device__ __forceinline__ double2 f2(const double a, const double b) { return make_double2(a, b); }
-__device__ __forceinline__ double2 f2s(const double a) { return make_double2(a, a); }
-__device__ __forceinline__ double2 add2(const double2 a, const double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 sub2(const double2 a, const double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ double2 mul2(const double2 a, const double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
-__device__ __forceinline__ double2 fma2(const double2 a, const double2 b, const double2 c) { return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y)); }
-__device__ __forceinline__ double2 rcp2(const double2 a) { return make_double2(rcp_f64(a.x), rcp_f64(a.y)); }
-__device__ __forceinline__ double blend2(const double2 w, const double2 F) { const double2 t = mul2(F, w); return t.x + t.y; }
-// the pair type of a value type
-template <class T> struct PairOf;
-template <> struct PairOf<float>  { typedef float2 V; };
-template <> struct PairOf<double> { typedef double2 V; };
+__device__ __forceinline__ float  add_(const float a, const float b)   { return __fadd_rn(a, b); }
+__device__ __forceinline__ float  sub_(const float a, const float b)   { return __fsub_rn(a, b); }
+__device__ __forceinline__ float  mul_(const float a, const float b)   { return __fmul_rn(a, b); }
+__device__ __forceinline__ float  fma_(const float a, const float b, const float c)    { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double add_(const double a, const double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double sub_(const double a, const double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ double mul_(const double a, const double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double fma_(const double a, const double b, const double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float2 add_(const float2 a, const float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 mul_(const float2 a, const float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 fma_(const float2 a, const float2 b, const float2 c) { return __ffma2_rn(a, b, c); }
+// a - b as one packed instruction (b * -1 is exact)
+__device__ __forceinline__ float2 sub_(const float2 a, const float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
+__device__ __forceinline__ float2 rcp_approx(const float2 a) { return make_float2(rcp_approx(a.x), rcp_approx(a.y)); }
+// a * b as one instruction per lane
+__device__ __forceinline__ float  mul1_(const float a, const float b)   { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul1_(const double a, const double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float2 mul1_(const float2 a, const float2 b) { return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)); }
+__device__ __forceinline__ float2 dsqrt(const float2 a) { return make_float2(dsqrt(a.x), dsqrt(a.y)); }
+__device__ __forceinline__ float2 dmin(const float2 a, const float2 b) { return make_float2(dmin(a.x, b.x), dmin(a.y, b.y)); }
+__device__ __forceinline__ float2 dmax(const float2 a, const float2 b) { return make_float2(dmax(a.x, b.x), dmax(a.y, b.y)); }
+// conditions of one value or of both lanes, and selection by them
+struct Bool2 { bool x, y; };
+template <class T> __device__ __forceinline__ bool not_negative(const T a) { return !(a < (T)0); }
+template <class T> __device__ __forceinline__ bool is_zero(const T a) { return a == (T)0; }
+template <class T> __device__ __forceinline__ T pick(const bool c, const T a, const T b) { return c ? a : b; }
+__device__ __forceinline__ Bool2 not_negative(const float2 a) { return Bool2{!(a.x < 0.0f), !(a.y < 0.0f)}; }
+__device__ __forceinline__ Bool2 is_zero(const float2 a) { return Bool2{a.x == 0.0f, a.y == 0.0f}; }
+__device__ __forceinline__ float2 pick(const Bool2 c, const float2 a, const float2 b) { return make_float2(c.x ? a.x : b.x, c.y ? a.y : b.y); }
+// the constant c in every lane
+template <class V> __device__ __forceinline__ V splat(const double c);
+template <> __device__ __forceinline__ float  splat<float>(const double c)  { return (float)c; }
+template <> __device__ __forceinline__ double splat<double>(const double c) { return c; }
+template <> __device__ __forceinline__ float2 splat<float2>(const double c) { return make_float2((float)c, (float)c); }
 
 // Minimum / maximum of three values in one operation (sm_100).
 __device__ __forceinline__ float min3f(const float a, const float b, const float c)
@@ -210,45 +266,86 @@ __device__ __forceinline__ float max3f(const float a, const float b, const float
 __device__ __forceinline__ double min3f(const double a, const double b, const double c) { return fmin(fmin(a, b), c); }
 __device__ __forceinline__ double max3f(const double a, const double b, const double c) { return fmax(fmax(a, b), c); }
 
-// Both edge values of one cell (fast policies), from the cell and its two
+// v clipped to [min, max] of three neighbours
+template <class T> __device__ __forceinline__ T clip3(const T v, const T a, const T b, const T c)
+{
+    return dmin(dmax(v, min3f(a, b, c)), max3f(a, b, c));
+}
+__device__ __forceinline__ float2 clip3(const float2 v, const float2 a, const float2 b, const float2 c)
+{
+    return make_float2(clip3(v.x, a.x, b.x, c.x), clip3(v.y, a.y, b.y, c.y));
+}
+
+// Edge values of one cell (fast policies), from the cell and its two
 // neighbours on either side, y0..y4 = cells l-2..l+2:
 //   R = value at the right edge l+1/2 (minus side of that face),
-//   L = value at the left edge l-1/2 (plus side of that face).
+//   L = value at the left edge l-1/2 (plus side of that face; kBoth only).
 // The Jiang-Shu smoothness indicators of the three sub-stencils
 // (l-2..l, l-1..l+1, l..l+2) integrate over cell l, so they are the same for
 // both edges (GPUonly.cuh:99-194 evaluates them again for every face): with
-//   k_j = y_j - 2 y_{j+1} + y_{j+2},  a_0 = y0-4y1+3y2, a_1 = y1-y3,
-//   a_2 = 3y2-4y3+y4,  g_j = 1/(13/3 k_j^2 + a_j^2 + 4 eps)^2
+// the differences d_i = y_{i+1} - y_i,
+//   k_j = d_{j+1} - d_j,  a_0 = k0 + 2 d1,  a_1 = d1 + d2,  a_2 = k2 - 2 d2,
+//   J_j = 13/3 k_j^2 + a_j^2 + 4 eps,  g_j = 1/J_j^2
 // (the indicators times 12/3, a common factor that cancels), the two edges
 // weigh them with mirrored linear weights d = (1, 6, 3):
-//   R = (y2+y3)/2 - k1/6 + (g0 (k0-k1)/3 + g2 (k1-k2)/2) / (g0 + 6 g1 + 3 g2)
-//   L = (y2+y1)/2 - k1/6 - (g2 (k1-k2)/3 + g0 (k0-k1)/2) / (3 g0 + 6 g1 + g2)
-// and both are clipped to [min, max] of y1, y2, y3.  Lane x of every pair
-// is the right edge, lane y the left edge.
-// The same algebra serves the fast FP64 form (T = double, lane by lane).
-template <class T>
-__device__ __forceinline__ void weno_cell_packed(const T y0, const T y1, const T y2,
-                                                 const T y3, const T y4, T& R, T& L)
+//   R = y2 + d2/2 - k1/6 + (g0 (k0-k1)/3 + g2 (k1-k2)/2) / (g0 + 6 g1 + 3 g2)
+//   L = y2 - d1/2 - k1/6 - (g2 (k1-k2)/3 + g0 (k0-k1)/2) / (3 g0 + 6 g1 + g2)
+// and both are clipped to [min, max] of y1, y2, y3.  Reversing y0..y4 turns R
+// into L bit for bit (every operation has its mirror image), so a ghost cell
+// whose left edge is wanted is reconstructed as the right edge of its
+// mirrored stencil.  In double (kShared) the weights are multiplied through
+// by J0^2 J1^2 J2^2 and the two sums share one reciprocal: one reciprocal
+// with its four Newton operations instead of five.  That holds up to
+// differences of about 1e18; beyond (the product of the sums out of range)
+// the result is false and the caller takes the form with five.
+template <bool kBoth, bool kShared, class V>
+__device__ __forceinline__ bool weno_edges(const V y0, const V y1, const V y2, const V y3, const V y4, V& R, V& L)
 {
-    typedef typename PairOf<T>::V V;
-    constexpr T e4 = (T)(4.0 * MPCF_WENOEPS);
-    const V Y04 = f2(y0, y4), Y13 = f2(y1, y3), Y22 = f2s(y2);
-    const V K02 = fma2(Y13, f2s((T)-2), add2(Y04, Y22));                        // (k0, k2)
-    const T k1  = fma(y2, (T)-2, y1 + y3);
-    const V A02 = fma2(Y22, f2s((T)3), fma2(Y13, f2s((T)-4), Y04));             // (a0, a2)
-    const T a1  = y1 - y3;
-    const V J02 = fma2(mul2(K02, f2s((T)13 / (T)3)), K02, fma2(A02, A02, f2s(e4)));
-    const T j1  = fma(k1 * ((T)13 / (T)3), k1, fma(a1, a1, e4));
-    const V G02 = rcp2(mul2(J02, J02));                                         // (g0, g2)
-    const T g1  = rcp_approx(j1 * j1);
-    const V den = fma2(f2(G02.y, G02.x), f2s((T)3), fma2(f2s(g1), f2s((T)6), G02));
-    const V E   = mul2(G02, f2(K02.x - k1, k1 - K02.y));                        // (g0 D0, g2 D2)
-    const V num = fma2(E, f2((T)1 / (T)3, -(T)1 / (T)3), mul2(f2(E.y, E.x), f2((T)0.5, (T)-0.5)));
-    const V p1  = fma2(f2s(k1), f2s(-(T)1 / (T)6), mul2(add2(Y22, f2(y3, y1)), f2s((T)0.5)));
-    const V r   = fma2(num, rcp2(den), p1);
-    const T lo = min3f(y1, y2, y3), hi = max3f(y1, y2, y3);
-    R = dmin(dmax(r.x, lo), hi);
-    L = dmin(dmax(r.y, lo), hi);
+    const V d0 = sub_(y1, y0), d1 = sub_(y2, y1), d2 = sub_(y3, y2), d3 = sub_(y4, y3);
+    const V k0 = sub_(d1, d0), k1 = sub_(d2, d1), k2 = sub_(d3, d2);
+    const V a0 = fma_(d1, splat<V>(2), k0), a1 = add_(d1, d2), a2 = fma_(d2, splat<V>(-2), k2);
+    const V c13 = splat<V>(13. / 3.), e4 = splat<V>(4. * MPCF_WENOEPS);
+    const V J0 = fma_(mul_(k0, c13), k0, fma_(a0, a0, e4));
+    const V J1 = fma_(mul_(k1, c13), k1, fma_(a1, a1, e4));
+    const V J2 = fma_(mul_(k2, c13), k2, fma_(a2, a2, e4));
+    V g0, g1, g2;
+    if constexpr (kShared)
+    {
+        const V p12 = mul_(J1, J2), p02 = mul_(J0, J2), p01 = mul_(J0, J1);
+        g0 = mul_(p12, p12); g1 = mul_(p02, p02); g2 = mul_(p01, p01);
+    }
+    else
+    {
+        g0 = rcp_approx(mul_(J0, J0)); g1 = rcp_approx(mul_(J1, J1)); g2 = rcp_approx(mul_(J2, J2));
+    }
+    const V E0 = mul_(g0, sub_(k0, k1)), E2 = mul_(g2, sub_(k1, k2));
+    const V denR = fma_(g2, splat<V>(3), fma_(g1, splat<V>(6), g0));
+    const V numR = fma_(E0, splat<V>(1. / 3.), mul_(E2, splat<V>(0.5)));
+    const V b = fma_(k1, splat<V>(-1. / 6.), y2);
+    const V pR = fma_(d2, splat<V>(0.5), b);
+    if constexpr (kShared)
+    {
+        const V denL = fma_(g0, splat<V>(3), fma_(g1, splat<V>(6), g2));
+        const V den = mul_(denR, denL), inv = rcp_approx(den);
+        R = clip3(fma_(mul_(numR, denL), inv, pR), y1, y2, y3);
+        if constexpr (kBoth)
+        {
+            const V numL = fma_(E2, splat<V>(-1. / 3.), mul_(E0, splat<V>(-0.5)));
+            L = clip3(fma_(mul_(numL, denR), inv, fma_(d1, splat<V>(-0.5), b)), y1, y2, y3);
+        }
+        return in_range(den, 0x1p-960, 0x1p960);
+    }
+    else
+    {
+        R = clip3(fma_(numR, rcp_approx(denR), pR), y1, y2, y3);
+        if constexpr (kBoth)
+        {
+            const V denL = fma_(g0, splat<V>(3), fma_(g1, splat<V>(6), g2));
+            const V numL = fma_(E2, splat<V>(-1. / 3.), mul_(E0, splat<V>(-0.5)));
+            L = clip3(fma_(numL, rcp_approx(denL), fma_(d1, splat<V>(-0.5), b)), y1, y2, y3);
+        }
+        return true;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -270,13 +367,9 @@ __device__ __forceinline__ typename Pol::T hllc_blend(const int s, const typenam
         return (T)(0.5f*(1 + s)) * L + (T)(0.5f*(1 - s)) * R;
 }
 
-// Everything one face produces.
-template <class T>
-struct FaceOut
-{
-    T f[7];      // fluxes rho, rho u, rho v, rho w, E, G, P
-    T Gm, Gp, Pm, Pp, vel;
-};
+// What one face gives its two cells: the fluxes of rho, rho u, rho v, rho w,
+// E, G, P and, last, the extra-term velocity.
+constexpr int kFaceOut = 8;
 
 // The face state after reconstruction: m = left (minus), p = right (plus).
 // n = normal velocity, t1/t2 = the transverse velocities in the order the
@@ -293,7 +386,7 @@ struct FaceState
 // instance of this code serves all three directions (the face pipeline is
 // ~1000 instructions; one copy keeps it resident in the instruction cache).
 template <class Pol>
-__device__ __forceinline__ void hllc_face(const FaceState<typename Pol::T>& S, const int dir, FaceOut<typename Pol::T>& o)
+__device__ __forceinline__ void hllc_face(const FaceState<typename Pol::T>& S, const int dir, typename Pol::T o[kFaceOut])
 {
     typedef typename Pol::T T;
     const T rm = S.rm, rp = S.rp, um = S.nm, up = S.np;
@@ -319,137 +412,136 @@ __device__ __forceinline__ void hllc_face(const FaceState<typename Pol::T>& S, c
     const T ss = (pp - pm + um*facm - up*facp) / (facm - facp);
 
     const int s = sign_star_of(ss);
-    const T s_minus = dmin((T)0.0f, sm);
-    const T s_pluss = dmax((T)0.0f, sp);
-    // every flux of this face divides by the same two denominators with the
-    // same normal velocities, so chi* is shared (identical operations)
-    const T chi_m = (sm - um) / (sm - ss);
-    const T chi_p = (sp - up) / (sp - ss);
-
-    // rho, G, P (passive): _hllc_rho (GPUonly.cuh:869-903)
+    // The blend (1+s)/2 L + (1-s)/2 R of a flux's two sides is 1*L + 0*R or
+    // 0*L + 1*R unless s* is exactly 0, so only the upwind side is evaluated
+    // (one pass, weight 1: the same value); at s = 0 a second pass evaluates
+    // the other side and both are blended as the reference does.  The other
+    // side's transverse velocities still enter as 0*t: a NaN or an infinity
+    // there reaches the fluxes as it does in the reference's sum (any other
+    // non-finite quantity makes s*, and with it everything, NaN).
+    const T z1 = (T)0 * (s < 0 ? S.t1m : S.t1p), z2 = (T)0 * (s < 0 ? S.t2m : S.t2p);
+#pragma unroll 1
+    for (int side = s < 0 ? 1 : 0; ; side = 1)
     {
-        const T qdm = rm*chi_m - rm, qdp = rp*chi_p - rp;
-        o.f[0] = hllc_blend<Pol, true>(s, rm*um + s_minus*qdm, rp*up + s_pluss*qdp);
+        const bool left = side == 0;
+        const T r = left ? rm : rp, u = left ? um : up, p = left ? pm : pp;
+        const T G = left ? Gm : Gp, P = left ? Pm : Pp;
+        const T t1 = left ? S.t1m : S.t1p, t2 = left ? S.t2m : S.t2p;
+        const T sk = left ? sm : sp;
+        const T sc = left ? dmin((T)0.0f, sm) : dmax((T)0.0f, sp);
+        const T du = sk - u;
+        // every flux of this face divides by the same denominator with the
+        // same normal velocity, so chi* is shared (identical operations)
+        const T chi = du / (sk - ss);
+        T f[kFaceOut];
+        // rho, G, P (passive): _hllc_rho (GPUonly.cuh:869-903)
+        const T q0 = r*u;
+        f[0] = q0 + sc*(r*chi - r);
+        f[5] = G*u + sc*(G*chi - G);
+        f[6] = P*u + sc*(P*chi - P);
+        // normal momentum: _hllc_pvel (GPUonly.cuh:947-984)
+        const T fn = (q0*u + p) + sc*(r*ss*chi - q0);
+        // transverse momenta: _hllc_vel (GPUonly.cuh:906-944)
+        const T q1 = r*t1, q2 = r*t2;
+        const T ft1 = q1*u + sc*(q1*chi - q1);
+        const T ft2 = q2*u + sc*(q2*chi - q2);
+        // energy: _hllc_e (GPUonly.cuh:987-1026)
+        {
+            const T q = G*p + P + (T)0.5f*r*(u*u + t1*t1 + t2*t2);
+            f[4] = u*(q + p) + sc*(chi*(q + (ss - u)*(r*ss + p/du)) - q);
+        }
+        // extra-term velocity: _extraterm_hllc_vel (GPUonly.cuh:1029-1042)
+        f[7] = u + sc*(chi - (T)1.0f);
+        // normal / transverse momenta back to (rho u, rho v, rho w):
+        // x: (n, t1, t2), y: (t1, n, t2), z: (t1, t2, n)
+        f[1] = dir == 0 ? fn : ft1;
+        f[2] = dir == 1 ? fn : (dir == 0 ? ft1 : ft2);
+        f[3] = dir == 2 ? fn : ft2;
+        if (s != 0)
+        {
+#pragma unroll
+            for (int m = 0; m < kFaceOut; ++m) o[m] = f[m];
+            o[1] = o[1] + (dir == 0 ? (T)0 : z1);
+            o[2] = o[2] + (dir == 1 ? (T)0 : (dir == 0 ? z1 : z2));
+            o[3] = o[3] + (dir == 2 ? (T)0 : z2);
+            o[4] = o[4] + (z1 + z2);
+            return;
+        }
+        if (side)
+        {
+#pragma unroll
+            for (int m = 0; m < kFaceOut; ++m)
+                o[m] = (m == 0 || m == 5 || m == 6) ? hllc_blend<Pol, true>(0, o[m], f[m]) : hllc_blend<Pol, false>(0, o[m], f[m]);
+            return;
+        }
+#pragma unroll
+        for (int m = 0; m < kFaceOut; ++m) o[m] = f[m];
     }
-    {
-        const T qdm = Gm*chi_m - Gm, qdp = Gp*chi_p - Gp;
-        o.f[5] = hllc_blend<Pol, true>(s, Gm*um + s_minus*qdm, Gp*up + s_pluss*qdp);
-    }
-    {
-        const T qdm = Pm*chi_m - Pm, qdp = Pp*chi_p - Pp;
-        o.f[6] = hllc_blend<Pol, true>(s, Pm*um + s_minus*qdm, Pp*up + s_pluss*qdp);
-    }
-    // normal momentum: _hllc_pvel (GPUonly.cuh:947-984)
-    T fn;
-    {
-        const T qm = rm*um, qp = rp*up;
-        const T qdm = rm*ss*chi_m - qm, qdp = rp*ss*chi_p - qp;
-        fn = hllc_blend<Pol, false>(s, (qm*um + pm) + s_minus*qdm, (qp*up + pp) + s_pluss*qdp);
-    }
-    // transverse momenta: _hllc_vel (GPUonly.cuh:906-944)
-    T ft1, ft2;
-    {
-        const T qm = rm*S.t1m, qp = rp*S.t1p;
-        const T qdm = qm*chi_m - qm, qdp = qp*chi_p - qp;
-        ft1 = hllc_blend<Pol, false>(s, qm*um + s_minus*qdm, qp*up + s_pluss*qdp);
-    }
-    {
-        const T qm = rm*S.t2m, qp = rp*S.t2p;
-        const T qdm = qm*chi_m - qm, qdp = qp*chi_p - qp;
-        ft2 = hllc_blend<Pol, false>(s, qm*um + s_minus*qdm, qp*up + s_pluss*qdp);
-    }
-    // energy: _hllc_e (GPUonly.cuh:987-1026)
-    {
-        const T qm = Gm*pm + Pm + (T)0.5f*rm*(um*um + S.t1m*S.t1m + S.t2m*S.t2m);
-        const T qp = Gp*pp + Pp + (T)0.5f*rp*(up*up + S.t1p*S.t1p + S.t2p*S.t2p);
-        const T qdm = chi_m*(qm + (ss - um)*(rm*ss + pm/(sm - um))) - qm;
-        const T qdp = chi_p*(qp + (ss - up)*(rp*ss + pp/(sp - up))) - qp;
-        o.f[4] = hllc_blend<Pol, false>(s, um*(qm + pm) + s_minus*qdm, up*(qp + pp) + s_pluss*qdp);
-    }
-    // extra-term velocity: _extraterm_hllc_vel (GPUonly.cuh:1029-1042)
-    o.vel = hllc_blend<Pol, false>(s, um + s_minus*(chi_m - (T)1.0f), up + s_pluss*(chi_p - (T)1.0f));
-
-    // normal / transverse momenta back to (rho u, rho v, rho w):
-    // x: (n, t1, t2), y: (t1, n, t2), z: (t1, t2, n)
-    o.f[1] = dir == 0 ? fn : ft1;
-    o.f[2] = dir == 1 ? fn : (dir == 0 ? ft1 : ft2);
-    o.f[3] = dir == 2 ? fn : ft2;
-    o.Gm = Gm; o.Gp = Gp; o.Pm = Pm; o.Pp = Pp;
 }
 
-// The same face in the fast policies: every left/right-symmetric quantity is
-// one packed pair (lane x = minus / left, lane y = plus / right) and the
-// divisions are single-precision reciprocals.  The wave speeds follow
-// hllc_face above term by term; the fluxes are the same expressions
-// factored: the advected quantities share V = S (chi - 1) + u, and the
-// energy flux cancels the (s - u) of chi against the p/(s - u) of the
-// reference's star-state energy.
-template <class T>
-__device__ __forceinline__ void hllc_face_packed(const FaceState<T>& S, const int dir, FaceOut<T>& o)
+// The same face in the fast policies.  The wave speeds follow hllc_face above
+// term by term with approximate reciprocals.  The flux is then evaluated for
+// the upwind side alone (the sign of s* picks the side; at s* = 0 the two
+// sides' star fluxes agree), in the star state's own form: with
+// chi = (S - u)/(S - s*), S_ = min(0, S_left) or max(0, S_right) and
+//   w = s* chi  (S_ != 0: inside the fan)  or  u  (S_ = 0: supersonic)
+// the reference's F + S_ (U* - U) is
+//   X w for the advected quantities X, w itself for the extra-term velocity,
+//   rho (w u + (s* - u) S_ chi) + p          for the normal momentum,
+//   w (E + p + rho (s* - u) S_)              for the energy.
+// It needs half the operations of the two-sided blend, no division by S - u,
+// and is exactly 0 for the advected quantities when s* = 0.
+// V is one face, or a pair of faces (the y and x faces of a cell, each in its
+// own normal / transverse components).  Products that a sum follows directly
+// are formed lane by lane (mul1_): a packed product before a packed sum may
+// be contracted, and every face must come out the same from either form.
+template <class V> struct FaceFlux { V r, n, t1, t2, e, G, P, w; };
+
+template <class V>
+__device__ __forceinline__ void hllc_face_upwind(const FaceState<V>& S, FaceFlux<V>& o)
 {
-    typedef typename PairOf<T>::V V;
-    const V Rh = f2(S.rm, S.rp), Uh = f2(S.nm, S.np), Ph = f2(S.pm, S.pp);
-    const V Gh = f2(S.Gm, S.Gp), Qh = f2(S.Pm, S.Pp);
-    const V T1 = f2(S.t1m, S.t1p), T2 = f2(S.t2m, S.t2p);
-    const T um = S.nm, up = S.np;
-
+    const V um = S.nm, up = S.np;
     // Einfeldt bounds
-    const V ir = rcp2(Rh);
-    const T Rr   = dsqrt(S.rp * ir.x);
-    const T Rinv = rcp_approx((T)1 + Rr);
-    const V c2 = mul2(fma2(add2(Ph, Qh), rcp2(Gh), Ph), ir);
-    const T cm = dsqrt(c2.x), cp = dsqrt(c2.y);
-    const T eta_2 = (T)0.5 * Rr * Rinv * Rinv;
-    const T du = up - um;
-    const T d  = dsqrt((c2.x + Rr * c2.y) * Rinv + eta_2 * du * du);
-    const T uu = (um + Rr * up) * Rinv;
-    const T sm = dmin(uu - d, um - cm);
-    const T sp = dmax(uu + d, up + cp);
+    const V irm = rcp_approx(S.rm), irp = rcp_approx(S.rp);
+    const V cm2 = mul_(fma_(add_(S.pm, S.Pm), rcp_approx(S.Gm), S.pm), irm);
+    const V cp2 = mul_(fma_(add_(S.pp, S.Pp), rcp_approx(S.Gp), S.pp), irp);
+    const V cm = dsqrt(cm2), cp = dsqrt(cp2);
+    const V Rr   = dsqrt(mul_(S.rp, irm));
+    const V Rinv = rcp_approx(add_(splat<V>(1), Rr));
+    const V eta  = mul_(mul_(mul_(splat<V>(0.5), Rr), Rinv), Rinv);
+    const V du   = sub_(up, um);
+    const V d    = dsqrt(fma_(mul_(eta, du), du, mul_(fma_(Rr, cp2, cm2), Rinv)));
+    const V uu   = mul1_(fma_(Rr, up, um), Rinv);
+    const V sm = dmin(sub_(uu, d), sub_(um, cm));
+    const V sp = dmax(add_(uu, d), add_(up, cp));
 
-    // Batten star speed
-    const V SU  = sub2(f2(sm, sp), Uh);                       // (sm - um, sp - up)
-    const V fac = mul2(Rh, SU);
-    const T ss = (S.pp - S.pm + um * fac.x - up * fac.y) * rcp_approx(fac.x - fac.y);
-    const int s = sign_star_of(ss);
-    const V Sg  = f2(dmin((T)0, sm), dmax((T)0, sp));
-    const V SS  = f2s(ss);
-    const V Dinv = rcp2(sub2(f2(sm, sp), SS));                // 1/(s - s*)
-    const V D   = sub2(SS, Uh);                               // s* - u
-    const V C1  = mul2(D, Dinv);                              // chi - 1 = (s* - u)/(s - s*)
-    const V Wb  = f2((T)0.5 * (T)(1 + s), (T)0.5 * (T)(1 - s));
+    // Batten star speed (numerator and denominator with their signs changed)
+    const V um_s = sub_(um, sm), sp_u = sub_(sp, up);
+    const V fm = mul_(S.rm, um_s);
+    const V num = fma_(up, mul_(S.rp, sp_u), fma_(um, fm, sub_(S.pm, S.pp)));
+    const V ss = mul1_(num, rcp_approx(fma_(S.rp, sp_u, fm)));
 
-    // every advected quantity X has the star-state flux S (X chi - X) + X u
-    // = X V with V = S (chi - 1) + u, the extra-term velocity's argument too
-    const V A = mul2(Sg, C1);
-    const V V_ = add2(A, Uh);
-    // rho, G, P (passive)
-    o.f[0] = blend2(Wb, mul2(Rh, V_));
-    o.f[5] = blend2(Wb, mul2(Gh, V_));
-    o.f[6] = blend2(Wb, mul2(Qh, V_));
-    // normal momentum: S (rho s* chi - rho u) + rho u^2 + p
-    // = rho (S (s* chi - u) + u^2) + p
-    const V U2 = mul2(Uh, Uh);
-    // (s* chi - u = s* (chi - 1) + s* - u)
-    const T fn = blend2(Wb, fma2(Rh, fma2(Sg, fma2(SS, C1, D), U2), Ph));
-    // transverse momenta
-    const V RV = mul2(Rh, V_);
-    const T ft1 = blend2(Wb, mul2(T1, RV));
-    const T ft2 = blend2(Wb, mul2(T2, RV));
-    // energy: S (chi (Q + (s* - u)(rho s* + p/(s - u))) - Q) + u (Q + p)
-    // = Q V + S (s* - u)(rho s* (s - u) + p)/(s - s*) + u p, Q = E
-    {
-        const V ke = fma2(T2, T2, fma2(T1, T1, U2));
-        const V Q  = fma2(mul2(f2s((T)0.5), Rh), ke, fma2(Gh, Ph, Qh));
-        const V inner = fma2(mul2(Rh, SS), SU, Ph);
-        o.f[4] = blend2(Wb, fma2(Q, V_, fma2(A, inner, mul2(Uh, Ph))));
-    }
-    // extra-term velocity
-    o.vel = blend2(Wb, V_);
+    // the upwind side (left for s* >= 0, and for NaN, which then propagates)
+    const auto left = not_negative(ss);
+    const V r = pick(left, S.rm, S.rp), u = pick(left, um, up), p = pick(left, S.pm, S.pp);
+    const V t1 = pick(left, S.t1m, S.t1p), t2 = pick(left, S.t2m, S.t2p);
+    const V G = pick(left, S.Gm, S.Gp), P = pick(left, S.Pm, S.Pp);
+    const V s  = pick(left, sm, sp);
+    const V sc = pick(left, dmin(splat<V>(0), sm), dmax(splat<V>(0), sp));
 
-    o.f[1] = dir == 0 ? fn : ft1;
-    o.f[2] = dir == 1 ? fn : (dir == 0 ? ft1 : ft2);
-    o.f[3] = dir == 2 ? fn : ft2;
-    o.Gm = S.Gm; o.Gp = S.Gp; o.Pm = S.Pm; o.Pp = S.Pp;
+    const V chi = mul_(sub_(s, u), rcp_approx(sub_(s, ss)));
+    const V w   = pick(is_zero(sc), u, mul_(ss, chi));
+    const V X   = mul_(sub_(ss, u), sc);
+    const V ke  = fma_(t2, t2, fma_(t1, t1, mul_(u, u)));
+    const V E   = fma_(mul_(splat<V>(0.5), r), ke, fma_(G, p, P));
+    o.r  = mul_(r, w);
+    o.n  = fma_(mul_(r, X), chi, fma_(o.r, u, p));
+    o.t1 = mul_(t1, o.r);
+    o.t2 = mul_(t2, o.r);
+    o.e  = mul_(w, fma_(r, X, add_(E, p)));
+    o.G  = mul_(G, w);
+    o.P  = mul_(P, w);
+    o.w  = w;
 }
 
 // Both edge values of one cell with the reference's WENO3 reconstruction
@@ -496,16 +588,78 @@ __device__ __forceinline__ void weno_cell(const typename Pol::T y0, const typena
         typename Pol::T& R, typename Pol::T& L)
 {
     if constexpr (Pol::kWeno3)         weno3_cell_ref<Pol>(y1, y2, y3, R, L);
-    else if constexpr (Pol::kFastWeno) weno_cell_packed<typename Pol::T>(y0, y1, y2, y3, y4, R, L);
-    else                               weno_cell_ref<Pol>(y0, y1, y2, y3, y4, R, L);
+    else if constexpr (Pol::kFastWeno) weno_edges<true, false>(y0, y1, y2, y3, y4, R, L);
+    else                               weno_cell_ref<Pol, false>(y0, y1, y2, y3, y4, R, L);
 }
 
-// Wave speeds and fluxes of one face in the policy's arithmetic.
+// The same as a call, for the rare cells whose weights the forms without
+// branches (weno_cell_ref's, weno_edges' kShared) cannot take.
+template <class T> struct Edges { T R, L; };
 template <class Pol>
-__device__ __forceinline__ void face_hllc(const FaceState<typename Pol::T>& S, const int dir, FaceOut<typename Pol::T>& o)
+__device__ __noinline__ Edges<typename Pol::T> weno_cell_call(const typename Pol::T y0, const typename Pol::T y1,
+        const typename Pol::T y2, const typename Pol::T y3, const typename Pol::T y4)
 {
-    if constexpr (Pol::kFastWeno) hllc_face_packed<typename Pol::T>(S, dir, o);
-    else                          hllc_face<Pol>(S, dir, o);
+    Edges<typename Pol::T> e;
+    if constexpr (Pol::kFastWeno)
+    {
+        if (weno_edges<true, true>(y0, y1, y2, y3, y4, e.R, e.L)) return e;
+    }
+    weno_cell<Pol>(y0, y1, y2, y3, y4, e.R, e.L);
+    return e;
+}
+
+// The edge values m (minus side) and p (plus side) of a face, 7 primitives
+// each, in the face's components (x: normal u, transverse v, w; y: normal v,
+// transverse u, w; z: normal w, transverse u, v).
+template <class T>
+__device__ __forceinline__ void face_state(const T m[8], const T p[8], const int dir, FaceState<T>& S)
+{
+    S.rm = m[0]; S.rp = p[0];
+    S.nm  = dir == 0 ? m[1] : (dir == 1 ? m[2] : m[3]);  S.np  = dir == 0 ? p[1] : (dir == 1 ? p[2] : p[3]);
+    S.t1m = dir == 0 ? m[2] : m[1];                      S.t1p = dir == 0 ? p[2] : p[1];
+    S.t2m = dir == 2 ? m[2] : m[3];                      S.t2p = dir == 2 ? p[2] : p[3];
+    S.pm = m[4]; S.pp = p[4]; S.Gm = m[5]; S.Gp = p[5]; S.Pm = m[6]; S.Pp = p[6];
+}
+
+// Wave speeds and fluxes of the face between m and p in the policy's
+// arithmetic.
+template <class Pol>
+__device__ __forceinline__ void face_hllc(const typename Pol::T m[8], const typename Pol::T p[8], const int dir,
+                                          typename Pol::T o[kFaceOut])
+{
+    typedef typename Pol::T T;
+    FaceState<T> S;
+    face_state<T>(m, p, dir, S);
+    if constexpr (Pol::kFastWeno)
+    {
+        FaceFlux<T> f;
+        hllc_face_upwind<T>(S, f);
+        o[0] = f.r;
+        o[1] = dir == 0 ? f.n : f.t1;
+        o[2] = dir == 1 ? f.n : (dir == 0 ? f.t1 : f.t2);
+        o[3] = dir == 2 ? f.n : f.t2;
+        o[4] = f.e; o[5] = f.G; o[6] = f.P; o[7] = f.w;
+    }
+    else hllc_face<Pol>(S, dir, o);
+}
+
+// A y face and an x face at once, as the two lanes of a pair (the fast FP32
+// forms).
+__device__ __forceinline__ void face_hllc_yx(const float my[8], const float py[8], const float mx[8], const float px[8],
+                                             float oy[kFaceOut], float ox[kFaceOut])
+{
+    FaceState<float2> S;
+    S.rm  = make_float2(my[0], mx[0]); S.rp  = make_float2(py[0], px[0]);
+    S.nm  = make_float2(my[2], mx[1]); S.np  = make_float2(py[2], px[1]);
+    S.t1m = make_float2(my[1], mx[2]); S.t1p = make_float2(py[1], px[2]);
+    S.t2m = make_float2(my[3], mx[3]); S.t2p = make_float2(py[3], px[3]);
+    S.pm  = make_float2(my[4], mx[4]); S.pp  = make_float2(py[4], px[4]);
+    S.Gm  = make_float2(my[5], mx[5]); S.Gp  = make_float2(py[5], px[5]);
+    S.Pm  = make_float2(my[6], mx[6]); S.Pp  = make_float2(py[6], px[6]);
+    FaceFlux<float2> f;
+    hllc_face_upwind<float2>(S, f);
+    oy[0] = f.r.x; oy[1] = f.t1.x; oy[2] = f.n.x;  oy[3] = f.t2.x; oy[4] = f.e.x; oy[5] = f.G.x; oy[6] = f.P.x; oy[7] = f.w.x;
+    ox[0] = f.r.y; ox[1] = f.n.y;  ox[2] = f.t1.y; ox[3] = f.t2.y; ox[4] = f.e.y; ox[5] = f.G.y; ox[6] = f.P.y; ox[7] = f.w.y;
 }
 
 // Conserved (rho, rho u, rho v, rho w, E, G, P) -> primitives (rho, u, v, w,

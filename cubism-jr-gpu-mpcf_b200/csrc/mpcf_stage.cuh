@@ -11,29 +11,27 @@
 // PCIe streaming (GPUlab.cpp:202-372,703-793); all state stays in HBM.
 //
 // Work decomposition.  A tile is 32 x TY columns in x-y and a z-chunk of
-// depth dz.  Warp w < TY owns row w, one thread per column; for TY = 2^n - 1
-// a further warp (the helper) owns no column.  The CTA marches up the chunk
-// one slab at a time:
-//   * a 6-slab ring of primitives (rho,u,v,w,p,G,P) of the tile's own
-//     columns lives in shared memory (z-stencil of the z faces);
-//   * slab k with its 3-cell x/y halo is staged in `cur` (x/y stencils);
-//   * reconstruction is per cell: the three WENO5 smoothness indicators of
-//     a cell serve both its edge values (the minus side of the face right
-//     of it and the plus side of the face left of it), in every direction;
-//   * z: every column thread reconstructs its cell k, evaluates the z face
-//     k-1/2 from the carried upper edge of cell k-1, and finalises cell
-//     k-1: rhs = a*R - dtinvh*div(F) (with the G/P extra terms),
-//     R <- rhs, U_next <- b*rhs + U;
-//   * x, y: every column thread writes its cell's edge values into the face
-//     slots in shared memory; the helper warp reconstructs the ghost cells
-//     around the tile (rows -1 and TY, columns -1 and 32; without a helper
-//     warps 0..2 take one job each, or every warp a share of their planes
-//     in the reference-rounding forms); after a barrier each face is
-//     evaluated in place in its slot, the x face left of every cell and the
-//     y face below it by the cell's thread, the faces above and right of
-//     the tile by the helper (warps 3 and 4 without one);
-//   * after a second barrier every cell gathers its x/y flux differences,
-//     carried to its finalisation in the next slab.
+// depth dz.  Warp w owns row w, one thread per column.  The CTA marches up
+// the chunk one slab at a time, two phases and two barriers per slab k:
+//   I  the x/y flux differences of cell k-1 (its own faces in registers, the
+//      faces right of and above it from the neighbours); z: both edges of
+//      cell k, the face k-1/2 from them and the carried upper edge of cell
+//      k-1, and with it cell k-1 is finalised:
+//      rhs = a*R - dtinvh*div(F) (with the G/P extra terms), R <- rhs,
+//      U_next <- b*rhs + U;  then the y and x edges of cell k, and a share of
+//      the ghost edges around the tile (rows -1 and TY, columns -1 and 32);
+//   II the y face below and the x face left of cell k, two warps the faces
+//      above and right of the tile; the next slab's primitives (the cell's
+//      own column three slabs up, the tile's halo one slab up) are converted
+//      into shared memory.
+// Reconstruction is per cell: the three WENO smoothness indicators of a cell
+// serve both its edge values (the minus side of the face right of it and the
+// plus side of the face left of it), in every direction.  A face's edge
+// values and fluxes stay in the registers of the cell above / right of it;
+// what the neighbour needs goes through one shuffle in x (the right edge up,
+// the flux down) and through one slot of shared memory in y, which holds the
+// upper edge of the row below until the face is evaluated and its flux after.
+// The G/P sums of the extra terms need only the cell's own six edges.
 // Each cell is converted to primitives once per stage (the reference
 // converts the six stencil cells again at every face).  The state is
 // ping-ponged (read U[parity], write U[parity^1]) so neighbouring tiles
@@ -41,17 +39,28 @@
 //
 // Loads.  Without TMA every thread loads its cells with ordinary global
 // loads (the generic path, any domain shape).  With TMA (domains whose rows
-// are multiples of 16 bytes), one elected thread issues two bulk tensor
-// copies per slab into shared memory -- the 40 x (TY+6) halo box of the next
-// slab and the 32 x TY interior of the slab three ahead -- which land while
-// the current slab's faces are evaluated; out-of-domain cells of the staged
-// box are mapped to their mirror / clamp source inside the box.  Waits on
-// the copies are bounded: a copy that does not complete sets an error bit,
-// the CTA stops waiting for copies and carries on (its data are then stale,
-// never out of bounds), so a failed copy cannot stall the launch.
+// are multiples of 16 bytes), one elected thread issues four bulk tensor
+// copies per slab into shared memory: in phase I the 40 x (TY+6) halo box of
+// the next slab and the 32 x TY interior of the slab three ahead, which phase
+// II converts (out-of-domain cells of the staged box are mapped to their
+// mirror / clamp source inside the box); in phase II the register and the
+// state of the plane that the next phase I finalises.  Waits on the copies
+// are bounded: a copy that does not complete sets an error bit, the CTA stops
+// waiting for copies and carries on (its data are then stale, never out of
+// bounds), so a failed copy cannot stall the launch.
 //
 // DRAM traffic per cell-stage: read U (7 T) + read R (7 T) + write R and
 // U_next (14 T) = 112 B in FP32.  Halo and ring re-reads hit L2.
+//
+// What bounds it: instruction issue and the latency of dependent FP32
+// operations at 16 warps per SM (the mixed form: 1728 thread-instructions per
+// cell-stage, 62 % of the issue slots, FMA pipe 45 % and special-function
+// unit 46 % busy, DRAM 16 %).  512^3, 32 x 8 tiles, mixed: 28.9 ms a step
+// against 35.0 for one slab pass with face slots of 28 planes, three barriers
+// and two-sided fluxes; the parts: two phases, faces in registers, quantities
+// in packed pairs, upwind fluxes 32.8; halo addresses once per tile 30.6; the
+// row uniform to the compiler 30.0; y and x faces as a pair and the register
+// and state by bulk copy 28.9.
 #pragma once
 
 #include "mpcf_math.cuh"
@@ -63,47 +72,61 @@ constexpr int kTX = 32;
 
 __host__ __device__ constexpr size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// Shared-memory layout of one CTA.  The T region is addressed in elements.
-// Every primitive plane q (rho, u, v, w, p, G, P) has the same pitch kPP and
-// holds both stencil sources, so a stencil of any direction is
-// addr[j] + q*kPP with kPP a compile-time constant:
-//   plane q:  ring [6 slots][TY][32]      z-ring of the tile's own columns
-//             cur  [TY+6][38]             slab k with 3-cell x/y halos
-// Face slots, pitch kFP = (TY+1)*32, 14 planes each:
-//   fx   [14][TY][33]                     x faces of slab k
-//   fy   [14][TY+1][32]                   y faces of slab k
-// Before a face is evaluated, planes 0..6 of its slot hold its minus side
-// and planes 7..13 its plus side (the reconstructed edge values of the two
-// cells it separates); the evaluation overwrites planes 0..11 in place with
-// its results (7 fluxes, G-, G+, P-, P+, the extra-term velocity).
+// 16 bytes of T: the unit of the primitives' shared-memory planes.
+template <class T> struct Vec16;
+template <> struct Vec16<float>  { typedef float4 V; };
+template <> struct Vec16<double> { typedef double2 V; };
+
+__device__ __forceinline__ void unpack(const float4 v, float* q)   { q[0] = v.x; q[1] = v.y; q[2] = v.z; q[3] = v.w; }
+__device__ __forceinline__ void unpack(const double2 v, double* q) { q[0] = v.x; q[1] = v.y; }
+__device__ __forceinline__ float4  pack(const float* q)  { return make_float4(q[0], q[1], q[2], q[3]); }
+__device__ __forceinline__ double2 pack(const double* q) { return make_double2(q[0], q[1]); }
+
+// Shared-memory layout of one CTA.  A record of 8 values (the primitives rho,
+// u, v, w, p, G, P and a spare, or a face's 7 fluxes and its velocity) is
+// kVecs 16-byte vectors, vector v of every record in plane v, so that a warp
+// reads and writes whole records without bank conflicts in kVecs
+// instructions.  Inside a plane, in vectors:
+//   ring [5 slots][TY][32]   z-ring of the tile's own columns, slabs k-2..k+2
+//   cur  [TY+6][38]          slab k with 3-cell x/y halos
+//   y    [TY+1][32]          face below row j: the upper edge of the row below
+//                            (slot 0: of ghost row -1), then the face's flux
+//   top  [32]                lower edge of ghost row TY
+//   xg   [TY]                right edge of ghost column -1
+//   xr   [TY]                right edge of column 31, then the flux right of it
+//   xl   [TY]                left edge of ghost column 32
 // then, in bytes: the FP64 reduction scratch [TY][5], the tile broadcast,
-// two mbarriers and, with TMA, the two staging buffers (128-byte aligned):
+// three mbarriers and, with TMA, the staging buffers (128-byte aligned):
 //   A     [7][TY+6][40]                   halo box, x from x0-4, y from y0-3
 //   B     [7][TY][32]                     interior of a slab
+//   C     [2][7][TY][32]                  register and state of the plane
+//                                         that is finalised next
 template <class T, int TY, bool TMA>
 struct StageLayout
 {
-    static constexpr int kNF     = 14;                     // planes of a face slot
+    static constexpr int kVecs   = 8 * (int)sizeof(T) / 16;
+    static constexpr int kPer    = 16 / (int)sizeof(T);    // values per vector
     static constexpr int kCurW   = kTX + 6;                // cur row width
-    static constexpr int kRing   = TY * kTX;               // one ring slot of a plane
-    static constexpr int kCurOff = 6 * kRing;              // cur inside a plane
-    static constexpr int kPP     = kCurOff + (TY + 6) * kCurW;
-    static constexpr int kFP     = (TY + 1) * kTX;         // >= TY * 33 for TY <= 32
-    static constexpr int kFx     = 7 * kPP;
-    static constexpr int kFy     = kFx + kNF * kFP;
-    static constexpr int kEnd    = kFy + kNF * kFP;
+    static constexpr int kRing   = TY * kTX;               // one ring slot
+    static constexpr int kCurOff = 5 * kRing;
+    static constexpr int kYOff   = kCurOff + (TY + 6) * kCurW;
+    static constexpr int kTopOff = kYOff + (TY + 1) * kTX;
+    static constexpr int kXgOff  = kTopOff + kTX;
+    static constexpr int kXrOff  = kXgOff + TY;
+    static constexpr int kXlOff  = kXrOff + TY;
+    static constexpr int kPP     = (kXlOff + TY + 7) / 8 * 8;   // plane pitch
     static constexpr int kAW     = kTX + 8;                // staged halo box width
     static constexpr int kAH     = TY + 6;                 // staged halo box height
-    static constexpr size_t kRedBytes  = align_up(kEnd * sizeof(T), 16);
+    static constexpr size_t kRedBytes  = (size_t)kVecs * kPP * 16;
     static constexpr size_t kTileBytes = kRedBytes + sizeof(double) * TY * 5;
     static constexpr size_t kMbarBytes = align_up(kTileBytes + 16, 16);
     static constexpr size_t kABytes    = sizeof(T) * 7 * kAH * kAW;
     static constexpr size_t kBBytes    = sizeof(T) * 7 * TY * kTX;
-    static constexpr size_t kStageA    = align_up(kMbarBytes + 16, 128);
+    static constexpr size_t kStageA    = align_up(kMbarBytes + 32, 128);
     static constexpr size_t kStageB    = align_up(kStageA + kABytes, 128);
+    static constexpr size_t kStageC    = align_up(kStageB + kBBytes, 128);
     // + 128: the kernel rounds the dynamic shared-memory base up to 128 B
-    static constexpr size_t kBytes     = (TMA ? kStageB + kBBytes : kMbarBytes + 16) + 128;
-    static_assert(kFP >= TY * (kTX + 1), "x-face plane");
+    static constexpr size_t kBytes     = (TMA ? kStageC + 2 * kBBytes : kMbarBytes + 32) + 128;
 };
 
 // Boundary-condition map of one coordinate: absorbing clamps to the edge
@@ -211,6 +234,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
 // 2^18 polls, about 1.3 s on the B200 (a copy completes in microseconds).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
 {
+#pragma unroll 1
     for (int i = 0; i < (1 << 18); ++i)
         if (mbar_try_wait(bar, parity)) return true;
     return false;
@@ -237,45 +261,120 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* tmap, int 
                  :: "r"(dst), "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar) : "memory");
 }
 
-// Register budget: at least kMinWarpsPerSM resident warps per SM.  The
-// face pipeline has 14 independent reconstructions, so the compiler would
-// otherwise trade occupancy for unbounded instruction-level parallelism.
+// Register budget: at least kMinWarpsPerSM resident warps per SM (128
+// registers per thread).  The slab's 21 reconstructions are independent, so
+// the compiler would otherwise trade occupancy for unbounded
+// instruction-level parallelism (239 registers).
 // FP64 values take two registers, so its budget is half the warps.
 #ifndef MPCF_MIN_WARPS_PER_SM
 #define MPCF_MIN_WARPS_PER_SM 16
 #endif
-// Tile heights of the form 2^n - 1 (3, 7, 15) carry a helper warp that
-// takes the tile's extra jobs (ghost rows and columns, the faces above and
-// right of the tile); other heights (8) give them to warps 0..4, one each
-// (the reference-rounding forms spread the ghost reconstructions over all
-// warps), which suits domains whose y extents are multiples of 8.
-template <int TY> struct TileShape
-{
-    static constexpr bool kHelper = ((TY + 1) & TY) == 0;
-    static constexpr int kWarps = kHelper ? TY + 1 : TY;
-};
-
 template <class T, int TY> struct MinBlocks
 {
     static constexpr int w = sizeof(T) == 8 ? MPCF_MIN_WARPS_PER_SM / 2 : MPCF_MIN_WARPS_PER_SM;
-    static constexpr int v = (w / TileShape<TY>::kWarps) > 0 ? (w / TileShape<TY>::kWarps) : 1;
+    static constexpr int v = (w / TY) > 0 ? (w / TY) : 1;
 };
 
-// Threads of one CTA: TY column warps and, with a helper, the helper warp.
-template <int TY> __host__ __device__ constexpr int stage_threads() { return kTX * TileShape<TY>::kWarps; }
+// Threads of one CTA: a warp per row.
+template <int TY> __host__ __device__ constexpr int stage_threads() { return kTX * TY; }
 
-// Ghost job g of a tile (0: row -1, 1: row TY, 2: columns -1 and 32) for
-// lane tx: the centre of the stencil in the cur slab, its step, and the face
-// slot that takes the edge value (dR: a minus slot, from the right / upper
-// edge; dL: a plus slot, from the left / lower edge).  Columns -1 and 32
-// take lanes 0..TY-1 and 16..15+TY; false for the idle lanes.
-template <class L, int TY>
-__device__ __forceinline__ bool ghost_job(const int g, const int tx, int& base, int& step, int& dR, int& dL)
+// Record `i` (index of its vector in a plane) of 8 values, read / written.
+template <class T, int PP>
+__device__ __forceinline__ void ld8(const typename Vec16<T>::V* sm, const int i, T q[8])
 {
-    if (g == 0)      { base = L::kCurOff + 2 * L::kCurW + tx + 3;        step = L::kCurW; dR = L::kFy + tx; }
-    else if (g == 1) { base = L::kCurOff + (TY + 3) * L::kCurW + tx + 3; step = L::kCurW; dL = L::kFy + TY * kTX + tx; }
-    else if (tx < TY)                  { base = L::kCurOff + (tx + 3) * L::kCurW + 2;        step = 1; dR = L::kFx + tx * (kTX + 1); }
-    else if (tx >= 16 && tx < 16 + TY) { base = L::kCurOff + (tx - 13) * L::kCurW + kTX + 3; step = 1; dL = L::kFx + (tx - 16) * (kTX + 1) + kTX; }
+#pragma unroll
+    for (int v = 0; v < 8 * (int)sizeof(T) / 16; ++v) unpack(sm[i + v * PP], q + v * (16 / (int)sizeof(T)));
+}
+template <class T, int PP>
+__device__ __forceinline__ void st8(typename Vec16<T>::V* sm, const int i, const T q[8])
+{
+#pragma unroll
+    for (int v = 0; v < 8 * (int)sizeof(T) / 16; ++v) sm[i + v * PP] = pack(q + v * (16 / (int)sizeof(T)));
+}
+
+// Both edges of the cell whose stencil records are ad[0..4], all 7
+// quantities.  The fast FP32 forms take (rho, u), (v, w) and (p, G) as packed
+// pairs and P alone.
+template <class Pol, int PP>
+__device__ __forceinline__ void weno_record(const typename Vec16<typename Pol::T>::V* sm, const int ad[5],
+                                            typename Pol::T R[8], typename Pol::T L[8])
+{
+    typedef typename Pol::T T;
+    constexpr int kPer = 16 / (int)sizeof(T);
+    // The FP64 forms take their reciprocals without branches (reference
+    // rounding, 256^3: 20.5 against 23.3 ms a step).  In FP32, with half the registers
+    // per value, the longer live ranges spill as much as the branches cost
+    // (12.34 ms either way, 13.3 without the fences), so it keeps the
+    // compiler's division.
+    constexpr bool kBranchFree = sizeof(T) == 8 && !Pol::kWeno3;
+    bool ok = true;         // every quantity's weights are in that form's range
+#pragma unroll
+    for (int v = 0; v < 8 / kPer; ++v)
+    {
+        T y[5][kPer];
+#pragma unroll
+        for (int j = 0; j < 5; ++j) unpack(sm[ad[j] + v * PP], y[j]);
+#pragma unroll
+        for (int i = 0; i < kPer; i += (Pol::kFastWeno && kPer == 4) ? 2 : 1)
+        {
+            const int q = v * kPer + i;
+            if (q >= 7) continue;
+            if constexpr (Pol::kFastWeno && kPer == 4)
+            {
+                if (q < 6)
+                {
+                    float2 r, l;
+                    weno_edges<true, false>(make_float2(y[0][i], y[0][i + 1]), make_float2(y[1][i], y[1][i + 1]),
+                                     make_float2(y[2][i], y[2][i + 1]), make_float2(y[3][i], y[3][i + 1]),
+                                     make_float2(y[4][i], y[4][i + 1]), r, l);
+                    R[q] = r.x; R[q + 1] = r.y; L[q] = l.x; L[q + 1] = l.y;
+                    continue;
+                }
+            }
+            if constexpr (kBranchFree)
+            {
+                if constexpr (Pol::kFastWeno) ok &= weno_edges<true, true>(y[0][i], y[1][i], y[2][i], y[3][i], y[4][i], R[q], L[q]);
+                else                          ok &= weno_cell_ref<Pol, true>(y[0][i], y[1][i], y[2][i], y[3][i], y[4][i], R[q], L[q]);
+                // two quantities at a time: more overlap than this spills
+                // (fast form, 256^3: 11.5 ms a step, 13.1 without the fences)
+                if (q % 2 == (Pol::kFastWeno ? 0 : 1)) __syncwarp();
+            }
+            else
+                weno_cell<Pol>(y[0][i], y[1][i], y[2][i], y[3][i], y[4][i], R[q], L[q]);
+        }
+    }
+    if constexpr (kBranchFree)
+    {
+        if (!ok)
+        {
+            const T* smT = reinterpret_cast<const T*>(sm);
+#pragma unroll
+            for (int q = 0; q < 7; ++q)
+            {
+                const int off = q % kPer + q / kPer * (PP * kPer);
+                const Edges<T> e = weno_cell_call<Pol>(smT[ad[0] * kPer + off], smT[ad[1] * kPer + off], smT[ad[2] * kPer + off],
+                                                       smT[ad[3] * kPer + off], smT[ad[4] * kPer + off]);
+                R[q] = e.R;
+                L[q] = e.L;
+            }
+        }
+    }
+    R[7] = L[7] = (T)0;
+}
+
+// Ghost edges of a tile, job g: 0 the right (upper) edges of row -1, 1 the
+// left (lower) edges of row TY, 2 the right edges of column -1 (lanes
+// 0..TY-1) and the left edges of column 32 (lanes 16..15+TY).  base: the
+// stencil's centre record, step: to the next record towards the wanted edge
+// (a left edge is the right edge of the mirrored stencil), dst: the record
+// that takes the edge; false for the idle lanes.
+template <class L, int TY>
+__device__ __forceinline__ bool ghost_job(const int g, const int tx, int& base, int& step, int& dst)
+{
+    if (g == 0)      { base = L::kCurOff + 2 * L::kCurW + tx + 3;        step = L::kCurW;  dst = L::kYOff + tx; }
+    else if (g == 1) { base = L::kCurOff + (TY + 3) * L::kCurW + tx + 3; step = -L::kCurW; dst = L::kTopOff + tx; }
+    else if (tx < TY)                  { base = L::kCurOff + (tx + 3) * L::kCurW + 2;        step = 1;  dst = L::kXgOff + tx; }
+    else if (tx >= 16 && tx < 16 + TY) { base = L::kCurOff + (tx - 13) * L::kCurW + kTX + 3; step = -1; dst = L::kXlOff + tx - 16; }
     else return false;
     return true;
 }
@@ -286,59 +385,63 @@ stage_kernel(const StageArgs A)
 {
     typedef typename Pol::T T;
     typedef StageLayout<T, TY, TMA> L;
-#ifdef MPCF_CHECK_BOUNDS
-    // slot 0 of a face plane, x or y faces
-    auto face_slot = [](const int d) { return (d >= L::kFx && d < L::kFx + L::kFP) || (d >= L::kFy && d < L::kFy + L::kFP); };
-#endif
+    // the reference-rounding forms, short of registers, keep the lower y edge
+    // from phase I to phase II in the ring slot of slab k-2, free by then
+    constexpr bool kStashLy = !Pol::kFastWeno;
+    constexpr bool kPairFaces = Pol::kFastWeno && sizeof(T) == 4;   // the y and x faces as one packed pair
+    typedef typename Vec16<T>::V V;
     extern __shared__ __align__(16) unsigned char smem_dyn[];
     // 128-byte aligned base (bulk tensor copies need it for their targets)
     unsigned char* smem_raw = smem_dyn + ((128u - (smem_u32(smem_dyn) & 127u)) & 127u);
-    T* sm = reinterpret_cast<T*>(smem_raw);
+    V* sm = reinterpret_cast<V*>(smem_raw);
     double* red = reinterpret_cast<double*>(smem_raw + L::kRedBytes);
     int* tile_bc = reinterpret_cast<int*>(smem_raw + L::kTileBytes);
     const uint32_t barA = smem_u32(smem_raw + L::kMbarBytes);
-    const uint32_t barB = barA + 8;
+    const uint32_t barB = barA + 8, barC = barA + 16;
     T* stA = reinterpret_cast<T*>(smem_raw + L::kStageA);
     T* stB = reinterpret_cast<T*>(smem_raw + L::kStageB);
+    T* stC = reinterpret_cast<T*>(smem_raw + L::kStageC);
 
     const int tx = threadIdx.x & (kTX - 1);
-    const int ty = threadIdx.x >> 5;
+    // (the shuffle tells the compiler that the row is uniform over the warp)
+    const int ty = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     const T a = (T)A.a;
     const T b = (T)A.b;
     const T factor6 = (T)1.0f / (T)6.0f;   // GPUkernels.cu:1103
     bool ok = true;
     bool oob = false;                      // bounds-checking build: an index left its buffer
-    uint32_t phA = 0, phB = 0;             // mbarrier phase parities
-    __shared__ T sos_w[TileShape<TY>::kWarps];   // per-warp maxima of the fused sound speed
+    uint32_t phA = 0, phB = 0, phC = 0;    // mbarrier phase parities
+    __shared__ T sos_w[TY];                // per-warp maxima of the fused sound speed
     // A thread whose bounded wait runs out sets tma_late and waits for no
     // further copy.  Thread 0 issues every copy; once it has given up it
     // issues none, and before the CTA takes another tile or exits it waits
     // (bounded again) for its copies that no wait of its own has seen
     // complete: pendA/pendB, with the parity of that copy's phase.
     bool tma_late = false;
-    bool pendA = false, pendB = false;
-    uint32_t parA = 0, parB = 0;
+    bool pendA = false, pendB = false, pendC = false;
+    uint32_t parA = 0, parB = 0, parC = 0;
     bool tma_inflight = false;             // a drain wait ran out as well
-    // thread 0: one bulk copy into stage buffer `st` (barrier `bar`), with
-    // its phase recorded as pending (and counted in failure-detection tests)
+    // thread 0: one bulk copy of a slab into buffer A or B, with its phase
+    // recorded as pending (and counted in failure-detection tests)
     auto issue = [&](const char* tmap, const bool isA, const int c0, const int c1, const int c2)
     {
         if (isA) { mbar_expect_tx(barA, (uint32_t)L::kABytes); tma_load_4d(smem_u32(stA), tmap, c0, c1, c2, 0, barA); pendA = true; parA = phA; }
         else     { mbar_expect_tx(barB, (uint32_t)L::kBBytes); tma_load_4d(smem_u32(stB), tmap + 128, c0, c1, c2, 0, barB); pendB = true; parB = phB; }
         if (A.test_flags) atomicAdd(A.counter + 1, 1u);
     };
-    // bounded wait of this thread on `bar` for phase `ph`; thread 0 clears
-    // the copy's pending mark when it sees it complete
-    auto wait_copy = [&](const bool isA)
+    // bounded wait of this thread for the copy into buffer A, B or C (0, 1,
+    // 2); thread 0 clears the copy's pending mark when it sees it complete
+    auto wait_copy = [&](const int which)
     {
         if (tma_late) return;
-        if (!mbar_wait(isA ? barA : barB, isA ? phA : phB)) { tma_late = true; return; }
-        if (threadIdx.x == 0) { if (isA) pendA = false; else pendB = false; }
+        const uint32_t bar = which == 0 ? barA : (which == 1 ? barB : barC);
+        if (!mbar_wait(bar, which == 0 ? phA : (which == 1 ? phB : phC))) { tma_late = true; return; }
+        if (threadIdx.x == 0) { if (which == 0) pendA = false; else if (which == 1) pendB = false; else pendC = false; }
     };
 
     if (TMA)
     {
-        if (threadIdx.x == 0) { mbar_init(barA, 1); mbar_init(barB, 1); mbar_init_fence(); }
+        if (threadIdx.x == 0) { mbar_init(barA, 1); mbar_init(barB, 1); mbar_init(barC, 1); mbar_init_fence(); }
         __syncthreads();
     }
 
@@ -348,7 +451,7 @@ stage_kernel(const StageArgs A)
     {
         if (threadIdx.x == 0) *tile_bc = A.tile0 + (int)atomicAdd(A.counter, 1u);
         __syncthreads();
-        t = *tile_bc;
+        t = __shfl_sync(0xffffffffu, *tile_bc, 0);
     }
     else t = A.tile0 + blockIdx.x;
 
@@ -372,8 +475,10 @@ stage_kernel(const StageArgs A)
         T* __restrict__       R    = (T*)DD.Rx;
         const T dtinvh = ((const T*)A.dtinvh)[d];
         const bool use_tma = TMA && DD.tma_ok;
-        // tensor maps of the buffer read in this stage: halo box, interior box
-        const char* tm = (const char*)A.tmaps + ((size_t)d * 4 + (size_t)A.parity * 2) * 128;
+        // tensor maps of the buffer read in this stage (halo box, interior
+        // box) and of the register (interior box, own planes only)
+        const char* tm = (const char*)A.tmaps + ((size_t)d * 5 + (size_t)A.parity * 2) * 128;
+        const char* tmR = (const char*)A.tmaps + ((size_t)d * 5 + 4) * 128;
 
         const int lt = t - DD.tile_begin;
         const int bx = lt % DD.tiles_x;
@@ -383,188 +488,120 @@ stage_kernel(const StageArgs A)
         const int z0 = DD.zlo + bz * A.dz;
         const int z1 = min(z0 + A.dz, DD.zlo + DD.nz);
         const int gx = x0 + tx, gy = y0 + ty;
-        const bool row = ty < TY;          // a column thread (not the helper)
-        const bool valid = row && (gx < D.nx) && (gy < D.ny);
+        const bool valid = (gx < D.nx) && (gy < D.ny);
         const int own = ty * kTX + tx;     // own column inside a ring slot
         // the tile's columns are all inside the domain: its ring holds the
         // exact primitives of every cur interior cell
         const bool full = (x0 + kTX <= D.nx) && (y0 + TY <= D.ny);
         // the staged halo box needs no boundary mapping in x and y
         const bool inner = (x0 >= 4) && (x0 + kTX + 4 <= D.nx) && (y0 >= 3) && (y0 + TY + 3 <= D.ny);
-
-        // ---- prologue: slabs z0-3 .. z0+1 of the own column into the ring
-        for (int sl = z0 - 3; row && sl <= z0 + 1; ++sl)
+        // the own column's record in ring slot r; slab k-2+j is in slot
+        // r2 + j modulo 5 with r2 the slot of slab k-2
+        auto ring = [&](int r) { r = r < 5 ? r : r - 5; return MPCF_IN(r * L::kRing + own, 0, L::kCurOff); };
+        // thread 0: the copies that phase II of slab k converts: the interior
+        // of slab k+3 and the halo box of slab k+1
+        auto issue_for = [&](const int k)
         {
-            T q[7];
-            load_prim<Pol>(D, U, gx, gy, sl, q, oob);
-            const int slot = (sl + 6) % 6;
-            const int ri = MPCF_IN(slot * L::kRing + own, 0, L::kCurOff);
-#pragma unroll
-            for (int m = 0; m < 7; ++m) sm[m * L::kPP + ri] = q[m];
-        }
-        if (use_tma && threadIdx.x == 0 && !tma_late)
-        {
-            // first copies: halo box of slab z0 and interior of slab z0+2
             bool fz;
             fence_proxy_async();
-            issue(tm, true, x0 - 4, y0 - 3, bc_map(z0, D.nz, D.bc4, D.bc5, fz));
-            issue(tm, false, x0, y0, bc_map(z0 + 2, D.nz, D.bc4, D.bc5, fz));
+            // the failure-detection tests arm the barrier of a copy without
+            // issuing it: the chunk's last copy, or its first copy after the
+            // first slab's (then later waits find the CTA given up, and no
+            // further copy is issued)
+            const bool drop = !PERSIST && (((A.test_flags & TEST_DROP_LAST_COPY) && k + 1 == z1) ||
+                                           ((A.test_flags & TEST_DROP_MID_COPY) && k == z0));
+            if (drop) mbar_expect_tx(barB, (uint32_t)L::kBBytes);
+            else      issue(tm, false, x0, y0, bc_map(k + 3, D.nz, D.bc4, D.bc5, fz));
+            if (k + 1 < z1) issue(tm, true, x0 - 4, y0 - 3, bc_map(k + 1, D.nz, D.bc4, D.bc5, fz));
+        };
+        if (use_tma && threadIdx.x == 0 && !tma_late) issue_for(z0 - 1);
+
+        // ---- prologue: slabs z0-3 .. z0+1 of the own column into the ring
+#pragma unroll
+        for (int j = 0; j < 5; ++j)
+        {
+            T q[8];
+            load_prim<Pol>(D, U, gx, gy, z0 - 3 + j, q, oob);
+            q[7] = (T)0;
+            st8<T, L::kPP>(sm, ring(j), q);
         }
 
-        T Sp[7];                 // x/y part of the flux bracket of cell k-1
-        T sG = 0, sP = 0, dU = 0;
-        T zfp[12];               // z face (k-1)-1/2
-        T Rzp[7];                // per-cell z: right edge of cell k-1 (minus side of face k-1/2)
+        // halo cell i (0 .. 6*32 + 6*TY - 1: the cells the x/y stencils read;
+        // the corners are never read) at (lx, ly) relative to the tile
+        auto halo_place = [&](const int i, int& lx, int& ly)
+        {
+            if (i < 6 * kTX) { const int r = i >> 5; lx = i & (kTX - 1); ly = r < 3 ? r - 3 : TY + r - 3; }
+            else             { const int j = i - 6 * kTX, c = j % 6; ly = j / 6; lx = c < 3 ? c - 3 : kTX + c - 3; }
+        };
+        // its cell of the staged box, its record in cur and the momenta its
+        // boundary condition flips, packed: box | cur << 12 | fx << 30 | fy << 31
+        auto halo_cell = [&](const int lx, const int ly, const bool map)
+        {
+            bool fx = false, fy = false;
+            int mx = lx + 4, my = ly + 3;
+            if (map)
+            {
+                mx = min(max(bc_map(x0 + lx, D.nx, D.bc0, D.bc1, fx) - x0 + 4, 0), L::kAW - 1);
+                my = min(max(bc_map(y0 + ly, D.ny, D.bc2, D.bc3, fy) - y0 + 3, 0), L::kAH - 1);
+            }
+            return (unsigned)(my * L::kAW + mx) | (unsigned)(L::kCurOff + (ly + 3) * L::kCurW + lx + 3) << 12 |
+                   (fx ? 1u << 30 : 0u) | (fy ? 1u << 31 : 0u);
+        };
+        auto convert_halo = [&](const unsigned hc)
+        {
+            T c[7], q[8];
+            const int ai = MPCF_IN((int)(hc & 0xfffu), 0, L::kAH * L::kAW);
 #pragma unroll
-        for (int m = 0; m < 7; ++m) Sp[m] = 0;
+            for (int m = 0; m < 7; ++m) c[m] = stA[m * L::kAH * L::kAW + ai];
+            if (hc >> 30 & 1u) c[1] = -c[1];
+            if (hc >> 31)      c[2] = -c[2];
+            to_primitive<Pol>(c, q);
+            q[7] = (T)0;
+            st8<T, L::kPP>(sm, MPCF_IN((int)(hc >> 12 & 0x3ffffu), L::kCurOff, L::kYOff), q);
+        };
+        int hlx, hly;
+        halo_place(threadIdx.x, hlx, hly);
+        const unsigned hc0 = halo_cell(hlx, hly, !inner);
+        int kcur = 0;
+        auto convert_or_load = [&](const unsigned hc, const int i)
+        {
+            if (use_tma) { convert_halo(hc); return; }
+            int lx, ly;
+            halo_place(i, lx, ly);
+            T q[8];
+            load_prim<Pol>(D, U, x0 + lx, y0 + ly, kcur, q, oob);
+            q[7] = (T)0;
+            st8<T, L::kPP>(sm, MPCF_IN((int)(hc >> 12 & 0x3ffffu), L::kCurOff, L::kYOff), q);
+        };
+        // carried from slab to slab: the z face below, the upper z edge and
+        // the x/y faces left of / below the cell, the G/P sums of its edges
+        T zfp[8], Rz[8], Fx[8], Fy[8];
+        T sG = 0, sP = 0;
 #pragma unroll
-        for (int m = 0; m < 12; ++m) zfp[m] = 0;
+        for (int m = 0; m < 8; ++m) { zfp[m] = 0; Rz[m] = 0; Fx[m] = 0; Fy[m] = 0; }
         double cs[5] = {0, 0, 0, 0, 0};
         T smax = 0;              // fused sound speed of the new state (last stage)
         bool sbad = false;
 
-        for (int k = z0; k <= z1; ++k)
+        // lane l < 28 prefetches row piece l: field l % 7 of R / U, first / second line
+        const T* pf;
         {
-            // (A) leading slab k+2 of the own column
-            if (row)
-            {
-                const int slot = (k + 2 + 6) % 6;
-                T q[7];
-                if (use_tma)
-                {
-                    wait_copy(false);
-                    phB ^= 1;
-                    bool fx = false, fy = false, fz;
-                    int mx = tx, my = ty;
-                    if (!full)
-                    {
-                        mx = min(max(bc_map(gx, D.nx, D.bc0, D.bc1, fx) - x0, 0), kTX - 1);
-                        my = min(max(bc_map(gy, D.ny, D.bc2, D.bc3, fy) - y0, 0), TY - 1);
-                    }
-                    bc_map(k + 2, D.nz, D.bc4, D.bc5, fz);
-                    T c[7];
-                    const int bi = MPCF_IN(my * kTX + mx, 0, TY * kTX);
-#pragma unroll
-                    for (int m = 0; m < 7; ++m) c[m] = stB[m * TY * kTX + bi];
-                    if (fx) c[1] = -c[1];
-                    if (fy) c[2] = -c[2];
-                    if (fz) c[3] = -c[3];
-                    to_primitive<Pol>(c, q);
-                }
-                else load_prim<Pol>(D, U, gx, gy, k + 2, q, oob);
-                const int ri = MPCF_IN(slot * L::kRing + own, 0, L::kCurOff);
-#pragma unroll
-                for (int m = 0; m < 7; ++m) sm[m * L::kPP + ri] = q[m];
-            }
-            // (B) slab k with halos into cur (slab k < nz: no z mapping)
-            if (k < z1)
-            {
-                const int slot = k % 6;
-                if (use_tma && !full)
-                {
-                    // tile reaching past the domain: convert the whole staged
-                    // box, mapping out-of-domain cells to their sources
-                    wait_copy(true);
-                    phA ^= 1;
-                    for (int i = threadIdx.x; i < (TY + 6) * L::kCurW; i += stage_threads<TY>())
-                    {
-                        const int ly = i / L::kCurW - 3, lx = i % L::kCurW - 3;
-                        bool fx, fy;
-                        const int mx = min(max(bc_map(x0 + lx, D.nx, D.bc0, D.bc1, fx) - x0 + 4, 0), L::kAW - 1);
-                        const int my = min(max(bc_map(y0 + ly, D.ny, D.bc2, D.bc3, fy) - y0 + 3, 0), L::kAH - 1);
-                        T c[7], q[7];
-                        const int ai = MPCF_IN(my * L::kAW + mx, 0, L::kAH * L::kAW);
-#pragma unroll
-                        for (int m = 0; m < 7; ++m) c[m] = stA[m * L::kAH * L::kAW + ai];
-                        if (fx) c[1] = -c[1];
-                        if (fy) c[2] = -c[2];
-                        to_primitive<Pol>(c, q);
-                        const int ci = MPCF_IN(L::kCurOff + (ly + 3) * L::kCurW + lx + 3, L::kCurOff, L::kPP);
-#pragma unroll
-                        for (int m = 0; m < 7; ++m) sm[m * L::kPP + ci] = q[m];
-                    }
-                }
-                else
-                {
-                    // interior from the ring, then the 6*32 + 6*TY halo cells
-                    // the x/y stencils read (the corners are never read)
-                    if (row)
-                    {
-                        const int ci = MPCF_IN(L::kCurOff + (ty + 3) * L::kCurW + tx + 3, L::kCurOff, L::kPP);
-                        const int ri = MPCF_IN(slot * L::kRing + own, 0, L::kCurOff);
-#pragma unroll
-                        for (int m = 0; m < 7; ++m)
-                            sm[m * L::kPP + ci] = sm[m * L::kPP + ri];
-                    }
-                    if (use_tma)
-                    {
-                        wait_copy(true);
-                        phA ^= 1;
-                    }
-                    for (int i = threadIdx.x; i < 6 * kTX + 6 * TY; i += stage_threads<TY>())
-                    {
-                        int lx, ly;
-                        if (i < 6 * kTX)
-                        {
-                            const int r = i >> 5;
-                            lx = i & (kTX - 1);
-                            ly = r < 3 ? r - 3 : TY + r - 3;
-                        }
-                        else
-                        {
-                            const int j = i - 6 * kTX;
-                            const int c = j % 6;
-                            ly = j / 6;
-                            lx = c < 3 ? c - 3 : kTX + c - 3;
-                        }
-                        T q[7];
-                        if (use_tma)
-                        {
-                            bool fx = false, fy = false;
-                            int mx = lx + 4, my = ly + 3;
-                            if (!inner)
-                            {
-                                mx = min(max(bc_map(x0 + lx, D.nx, D.bc0, D.bc1, fx) - x0 + 4, 0), L::kAW - 1);
-                                my = min(max(bc_map(y0 + ly, D.ny, D.bc2, D.bc3, fy) - y0 + 3, 0), L::kAH - 1);
-                            }
-                            T c[7];
-                            const int ai = MPCF_IN(my * L::kAW + mx, 0, L::kAH * L::kAW);
-#pragma unroll
-                            for (int m = 0; m < 7; ++m) c[m] = stA[m * L::kAH * L::kAW + ai];
-                            if (fx) c[1] = -c[1];
-                            if (fy) c[2] = -c[2];
-                            to_primitive<Pol>(c, q);
-                        }
-                        else load_prim<Pol>(D, U, x0 + lx, y0 + ly, k, q, oob);
-                        const int ci = MPCF_IN(L::kCurOff + (ly + 3) * L::kCurW + lx + 3, L::kCurOff, L::kPP);
-#pragma unroll
-                        for (int m = 0; m < 7; ++m) sm[m * L::kPP + ci] = q[m];
-                    }
-                }
-            }
-            __syncthreads();
-            // the staging buffers are free again: copy the next slab's data
-            // while this slab's faces are evaluated
-            if (use_tma && threadIdx.x == 0 && !tma_late)
-            {
-                bool fz;
-                fence_proxy_async();
-                if (k + 1 <= z1)
-                {
-                    // the failure-detection tests arm the barrier of a copy
-                    // without issuing it: the chunk's last copy, or its
-                    // first copy after the prologue (then later waits find
-                    // the CTA given up, and no further copy is issued)
-                    const bool drop = !PERSIST && (((A.test_flags & TEST_DROP_LAST_COPY) && k + 1 == z1) ||
-                                                   ((A.test_flags & TEST_DROP_MID_COPY) && k == z0));
-                    if (drop) mbar_expect_tx(barB, (uint32_t)L::kBBytes);
-                    else      issue(tm, false, x0, y0, bc_map(k + 3, D.nz, D.bc4, D.bc5, fz));
-                }
-                if (k + 1 < z1) issue(tm, true, x0 - 4, y0 - 3, bc_map(k + 1, D.nz, D.bc4, D.bc5, fz));
-            }
+            const int f = tx % 7, w = tx / 7;
+            pf = ((w & 1) ? U : (const T*)R) + f * D.fs - (long long)D.nx * D.ny + (long long)D.nx * min(gy, D.ny - 1) + min(x0 + ((w & 2) ? 31 : 0), D.nx - 1);
+        }
+        // slab z0-1 gives its upper z edge only
+        int r2 = 0;
+#pragma unroll 1
+        for (int k = z0 - 1; ; ++k)
+        {
+            const bool xy = k >= z0 && k < z1;     // slab k has x and y faces
+            // the staging buffers are free again (phase II of slab k-1 is
+            // behind the barrier): copy while this slab is worked on
+            if (use_tma && threadIdx.x == 0 && !tma_late && xy) issue_for(k);
 
-            // R and U of cell k-1 are first prefetched into L1, so that its
-            // finalisation after the z face finds them.
+            // ---- phase I
+            // without bulk copies, R and U of cell k-1 are first prefetched
+            // into L1, so that its finalisation after the z face finds them
             const bool fin = (k > z0) && valid;
 #ifdef MPCF_CHECK_BOUNDS
             // cell k-1 of the own column: inside the domain's own planes
@@ -574,247 +611,362 @@ stage_kernel(const StageArgs A)
 #else
             const long long idx = (long long)gx + (long long)D.nx * ((long long)gy + (long long)D.ny * (k - 1));
 #endif
-            if (fin)
-            {
+            if (!use_tma && k > z0 && tx < 28) prefetch_l1(pf + (long long)D.nx * D.ny * k);
+            // x/y part of cell k-1: its own faces, the face right of it from
+            // the next lane (or the tile's extra face) and the face above it
+            // from its slot
+            T S[7], dU = 0;
 #pragma unroll
-                for (int m = 0; m < 7; ++m) { prefetch_l1(R + m * D.fs + idx); prefetch_l1(U + m * D.fs + idx); }
-            }
-            // (E) finalisation of cell k-1 of the own column from the z face
-            // k-1/2: rhs = a*R - dtinvh*div(F) (with the G/P extra terms),
-            // R <- rhs, U_next <- b*rhs + U.  It reads only this thread's
-            // registers and global memory.
-            auto finalize = [&](const FaceOut<T>& zf)
+            for (int m = 0; m < 7; ++m) S[m] = 0;
+            if (k > z0)
             {
-                T Rold[7], Uold[7];
+                T Fr[8], Fa[8];
 #pragma unroll
-                for (int m = 0; m < 7; ++m) { Rold[m] = R[m * D.fs + idx]; Uold[m] = __ldg(U + m * D.fs + idx); }
-                const T sumG = sG + (zfp[8] + zf.Gm);
-                const T sumP = sP + (zfp[10] + zf.Pm);
-                const T divU = dU + (zf.vel - zfp[11]);
-                T un[7];
+                for (int m = 0; m < 8; ++m) Fr[m] = __shfl_down_sync(0xffffffffu, Fx[m], 1);
+                if (tx == kTX - 1) ld8<T, L::kPP>(sm, L::kXrOff + ty, Fr);
+                ld8<T, L::kPP>(sm, L::kYOff + own + kTX, Fa);
 #pragma unroll
                 for (int m = 0; m < 7; ++m)
                 {
-                    T br = (Sp[m] + zf.f[m]) - zfp[m];
-                    if (m == 5) br = br - divU * sumG * factor6;
-                    if (m == 6) br = br - divU * sumP * factor6;
-                    const T rhs_m = dtinvh * br;
-                    const T rhs = a * Rold[m] - rhs_m;
-                    R[m * D.fs + idx] = rhs;
-                    un[m] = b * rhs + Uold[m];
-                    Un[m * D.fs + idx] = un[m];
+                    if constexpr (Pol::kFastWeno) S[m] = (Fr[m] - Fx[m]) + (Fa[m] - Fy[m]);
+                    else                          S[m] = ((Fr[m] - Fx[m]) + Fa[m]) - Fy[m];
                 }
-                ok = ok && physical<T>(un[0], un[4], un[5], un[6]);
-                if (A.sos_bits)
-                {
-                    const T v = cell_sos_rn<Pol>(un[0], un[1], un[2], un[3], un[4], un[5], un[6]);
-                    sbad = sbad || !(v >= (T)0);   // NaN (the maximum would drop it) or negative
-                    smax = dmax(smax, v);
-                }
-                if (SUMS)
-                {
-#pragma unroll
-                    for (int m = 0; m < 5; ++m) cs[m] += (double)un[m];
-                }
-            };
-            FaceOut<T> zf;
+                dU = (Fr[7] - Fx[7]) + (Fa[7] - Fy[7]);
+            }
+            // z: both edges of cell k, the face k-1/2, and cell k-1's
+            // finalisation: rhs = a*R - dtinvh*div(F) (with the G/P extra
+            // terms), R <- rhs, U_next <- b*rhs + U
+            T Rv[8], Lv[8];
             {
-                // (C) per-cell reconstruction and faces of slab k.
-                //  1. z (column threads): the right edge of cell k-1 (first
-                //     slab of a chunk only; later it is carried), both edges
-                //     of cell k, the z face k-1/2 from them, then cell k-1 is
-                //     finalised;
-                //  2. x and y edges of the own cell into the face slots: the
-                //     right / upper edge to the minus side of the face right
-                //     of / above the cell, the left / lower edge to the plus
-                //     side of the face left of / below it.  The helper warp
-                //     (without one: warps 0..2, or all warps in shares)
-                //     reconstructs the ghost cells around the tile: row -1,
-                //     row TY, columns -1 and 32;
-                //  3. after a barrier, the x face left of the own cell and the
-                //     y face below it, each evaluated in place in its slot;
-                //     the helper (warps 3 and 4 without one) evaluates the y
-                //     faces above the tile and the x faces right of it.  Without
-                //     a helper no warp takes more than one of the extra jobs,
-                //     which keeps the warps even at the barriers.
-                constexpr bool kHelper = TileShape<TY>::kHelper;
-                static_assert(TY <= 16, "ghost columns -1 and 32 take lanes 0..TY-1 and 16..15+TY");
-                static_assert(kHelper || TY >= 5, "without a helper, warps 0..4 take the extra jobs");
-                if (row)
+                int ad[5];
+#pragma unroll
+                for (int j = 0; j < 5; ++j) ad[j] = ring(r2 + j);
+                weno_record<Pol, L::kPP>(sm, ad, Rv, Lv);
+            }
+            if (k >= z0)
+            {
+                T zf[8];
+                face_hllc<Pol>(Rz, Lv, 2, zf);
+                if (use_tma && k > z0)
                 {
-#pragma unroll 1
-                    for (int cz = (k == z0) ? k - 1 : k; cz <= k; ++cz)
-                    {
-                        // ring slots of slabs cz-2 .. cz+2
-                        const int zs = (cz + 4) % 6;
-                        int ad[5];
-#pragma unroll
-                        for (int j = 0; j < 5; ++j) ad[j] = MPCF_IN((zs + j < 6 ? zs + j : zs + j - 6) * L::kRing + own, 0, L::kCurOff);
-                        T Rv[7], Lv[7];
-#pragma unroll
-                        for (int q = 0; q < 7; ++q)
-                        {
-                            const T* pl = sm + q * L::kPP;
-                            weno_cell<Pol>(pl[ad[0]], pl[ad[1]], pl[ad[2]], pl[ad[3]], pl[ad[4]], Rv[q], Lv[q]);
-                        }
-                        if (cz == k)
-                        {
-                            // z: normal w, transverse u, v
-                            FaceState<T> S;
-                            S.rm = Rzp[0]; S.rp = Lv[0]; S.nm = Rzp[3]; S.np = Lv[3];
-                            S.t1m = Rzp[1]; S.t1p = Lv[1]; S.t2m = Rzp[2]; S.t2p = Lv[2];
-                            S.pm = Rzp[4]; S.pp = Lv[4]; S.Gm = Rzp[5]; S.Gp = Lv[5]; S.Pm = Rzp[6]; S.Pp = Lv[6];
-                            face_hllc<Pol>(S, 2, zf);
-                        }
-#pragma unroll
-                        for (int q = 0; q < 7; ++q) Rzp[q] = Rv[q];
-                    }
-                    if (fin) finalize(zf);
-#pragma unroll
-                    for (int m = 0; m < 7; ++m) zfp[m] = zf.f[m];
-                    zfp[7] = zf.Gm; zfp[8] = zf.Gp; zfp[9] = zf.Pm; zfp[10] = zf.Pp; zfp[11] = zf.vel;
+                    wait_copy(2);
+                    phC ^= 1;
                 }
-                // the fast forms run the x/y loops unrolled by two (both loops:
-                // 3% faster at 512^3); the reference-rounding forms, with their
-                // double-promoted weights, keep one copy of each
-                constexpr int kXYUnroll = Pol::kFastWeno ? 2 : 1;
-                if (k < z1)
+                if (fin)
                 {
-                    // Own cells (x, then y) and the three ghost jobs: with a
-                    // helper, the helper warp takes them whole (it has no z
-                    // part); without one, in the fast forms warps 0..2 take
-                    // one each, and in the other forms every warp takes a
-                    // share of their 21 planes (below).
-                    constexpr bool kSplitGhosts = !kHelper && !Pol::kFastWeno;
-                    const int nr = row ? ((!kHelper && !kSplitGhosts && ty < 3) ? 3 : 2) : 3;
-#pragma unroll kXYUnroll
-                    for (int j = 0; j < nr; ++j)
+                    T Rold[7], Uold[7];
+                    if (use_tma)
                     {
-                        int base, step, dR = -1, dL = -1;
-                        if (row && j < 2)
-                        {
-                            // own cell: j = 0 x, j = 1 y
-                            base = L::kCurOff + (ty + 3) * L::kCurW + tx + 3;
-                            step = j ? L::kCurW : 1;
-                            dL = j ? L::kFy + ty * kTX + tx : L::kFx + ty * (kTX + 1) + tx;
-                            dR = j ? dL + kTX : dL + 1;
-                        }
-                        else if (!ghost_job<L, TY>(row ? ty : j, tx, base, step, dR, dL)) continue;
-#ifdef MPCF_CHECK_BOUNDS
-                        if (base - 2 * step < L::kCurOff || base + 2 * step >= L::kPP) { oob = true; base = L::kCurOff + 2 * step; }
-                        if (dR >= 0 && !face_slot(dR)) { oob = true; dR = -1; }
-                        if (dL >= 0 && !face_slot(dL)) { oob = true; dL = -1; }
-#endif
-                        T Rv[7], Lv[7];
 #pragma unroll
-                        for (int q = 0; q < 7; ++q)
-                        {
-                            const T* pl = sm + q * L::kPP + base;
-                            weno_cell<Pol>(pl[-2 * step], pl[-step], pl[0], pl[step], pl[2 * step], Rv[q], Lv[q]);
-                        }
-                        if (dR >= 0)
-                        {
-#pragma unroll
-                            for (int q = 0; q < 7; ++q) sm[dR + q * L::kFP] = Rv[q];
-                        }
-                        if (dL >= 0)
-                        {
-#pragma unroll
-                            for (int q = 0; q < 7; ++q) sm[dL + (7 + q) * L::kFP] = Lv[q];
-                        }
+                        for (int m = 0; m < 7; ++m) { Rold[m] = stC[m * L::kRing + own]; Uold[m] = stC[(7 + m) * L::kRing + own]; }
                     }
-                    if constexpr (kSplitGhosts)
+                    else
                     {
-                        // The 21 planes of the ghost jobs (3 jobs x 7
-                        // quantities) in contiguous ranges over the warps
-                        // (TY = 8: warps 0..4 take 3, the others 2), so that no
-                        // warp reaches the barrier 7 planes after another.  In
-                        // the reference-rounding forms this is 5% faster at
-                        // TY = 8; the fast forms lose the independent chains of
-                        // a whole job and are 3% slower with it.
-                        constexpr int kPer = 21 / TY, kRem = 21 % TY;
-                        int gi = ty * kPer + (ty < kRem ? ty : kRem);
-                        const int ge = gi + kPer + (ty < kRem ? 1 : 0);
-#pragma unroll 1
-                        for (; gi < ge; ++gi)
-                        {
-                            const int g = gi >= 14 ? 2 : (gi >= 7 ? 1 : 0);
-                            const int q = gi - 7 * g;
-                            int base, step, dR = -1, dL = -1;
-                            if (!ghost_job<L, TY>(g, tx, base, step, dR, dL)) continue;
-#ifdef MPCF_CHECK_BOUNDS
-                            if (base - 2 * step < L::kCurOff || base + 2 * step >= L::kPP) { oob = true; base = L::kCurOff + 2 * step; }
-                            if (dR >= 0 && !face_slot(dR)) { oob = true; continue; }
-                            if (dL >= 0 && !face_slot(dL)) { oob = true; continue; }
-#endif
-                            const T* pl = sm + q * L::kPP + base;
-                            T rv, lv;
-                            weno_cell<Pol>(pl[-2 * step], pl[-step], pl[0], pl[step], pl[2 * step], rv, lv);
-                            // the right / upper edge fills a minus slot, the
-                            // left / lower edge a plus slot
-                            if (dR >= 0) sm[dR + q * L::kFP] = rv;
-                            else         sm[dL + (7 + q) * L::kFP] = lv;
-                        }
+#pragma unroll
+                        for (int m = 0; m < 7; ++m) { Rold[m] = R[m * D.fs + idx]; Uold[m] = __ldg(U + m * D.fs + idx); }
                     }
-                    __syncthreads();
-                    const int nh = row ? ((!kHelper && (ty == 3 || ty == 4)) ? 3 : 2) : 2;
-#pragma unroll kXYUnroll
-                    for (int j = 0; j < nh; ++j)
+                    const T divU = dU + (zf[7] - zfp[7]);
+                    T un[7];
+#pragma unroll
+                    for (int m = 0; m < 7; ++m)
                     {
-                        int src, dir;
-                        if (row && j < 2) { dir = j; src = j ? L::kFy + ty * kTX + tx : L::kFx + ty * (kTX + 1) + tx; }
+                        T br;
+                        if constexpr (Pol::kFastWeno) br = S[m] + (zf[m] - zfp[m]);
+                        else                          br = (S[m] + zf[m]) - zfp[m];
+                        if (m == 5) br = br - divU * sG * factor6;
+                        if (m == 6) br = br - divU * sP * factor6;
+                        const T rhs_m = dtinvh * br;
+                        const T rhs = a * Rold[m] - rhs_m;
+                        R[m * D.fs + idx] = rhs;
+                        un[m] = b * rhs + Uold[m];
+                        Un[m * D.fs + idx] = un[m];
+                    }
+                    ok = ok && physical<T>(un[0], un[4], un[5], un[6]);
+                    if (A.sos_bits)
+                    {
+                        const T v = cell_sos_rn<Pol>(un[0], un[1], un[2], un[3], un[4], un[5], un[6]);
+                        sbad = sbad || !(v >= (T)0);   // NaN (the maximum would drop it) or negative
+                        smax = dmax(smax, v);
+                    }
+                    if (SUMS)
+                    {
+#pragma unroll
+                        for (int m = 0; m < 5; ++m) cs[m] += (double)un[m];
+                    }
+                }
+#pragma unroll
+                for (int m = 0; m < 8; ++m) zfp[m] = zf[m];
+            }
+            if (k == z1) break;
+#pragma unroll
+            for (int m = 0; m < 8; ++m) Rz[m] = Rv[m];
+
+            T Ly[8], Rx[8], Lx[8];
+#pragma unroll
+            for (int m = 0; m < 8; ++m) { Ly[m] = 0; Rx[m] = 0; Lx[m] = 0; }
+            if (xy)
+            {
+                // y, then x edges of the own cell.  The fast forms unroll the
+                // two; the reference-rounding forms, whose reconstruction is
+                // five times the code, keep one copy.
+                const T szG = Lv[5] + Rv[5], szP = Lv[6] + Rv[6];
+                T syG = 0, syP = 0;
+                constexpr int kXYUnroll = Pol::kFastWeno ? 2 : 1;
+#pragma unroll kXYUnroll
+                for (int j = 0; j < 2; ++j)
+                {
+                    const int step = j ? 1 : L::kCurW;
+                    const int base = L::kCurOff + (ty + 3) * L::kCurW + tx + 3;
+                    int ad[5];
+#pragma unroll
+                    for (int i = 0; i < 5; ++i) ad[i] = MPCF_IN(base + (i - 2) * step, L::kCurOff, L::kYOff);
+                    weno_record<Pol, L::kPP>(sm, ad, Rv, Lv);
+                    if (j == 0)
+                    {
+                        st8<T, L::kPP>(sm, L::kYOff + own + kTX, Rv);
+                        if constexpr (kStashLy) st8<T, L::kPP>(sm, ring(r2), Lv);
+#pragma unroll
+                        for (int m = 0; m < 7; ++m) Ly[m] = Lv[m];
+                        syG = Lv[5] + Rv[5];
+                        syP = Lv[6] + Rv[6];
+                    }
+                    else
+                    {
+                        if (tx == kTX - 1) st8<T, L::kPP>(sm, L::kXrOff + ty, Rv);
+#pragma unroll
+                        for (int m = 0; m < 7; ++m) { Rx[m] = Rv[m]; Lx[m] = Lv[m]; }
+                        sG = ((Lv[5] + Rv[5]) + syG) + szG;
+                        sP = ((Lv[6] + Rv[6]) + syP) + szP;
+                    }
+                }
+                // ghost edges around the tile, shared evenly by the warps
+                const T* smT = reinterpret_cast<const T*>(sm);
+                T* smTw = reinterpret_cast<T*>(sm);
+                if constexpr (Pol::kFastWeno && sizeof(T) == 4)
+                {
+                    // 14 jobs, 7 quantities of the two rows and 7 of the two
+                    // columns; a row / column and its mirror image on the
+                    // other side are the two lanes of a pair.  The rows'
+                    // jobs go to the first warps, the columns' to the last.
+                    auto edge_pair = [&](const int b0, const int s0, const int d0, const int b1, const int s1, const int d1, const int q)
+                    {
+                        const int off = (q & 3) + (q >> 2) * (L::kPP * 4);
+                        float a0[5], a1[5];
+#pragma unroll
+                        for (int i = 0; i < 5; ++i)
+                        {
+                            a0[i] = smT[MPCF_IN(b0 + (i - 2) * s0, L::kCurOff, L::kYOff) * 4 + off];
+                            a1[i] = smT[MPCF_IN(b1 + (i - 2) * s1, L::kCurOff, L::kYOff) * 4 + off];
+                        }
+                        float2 r, l;
+                        if (q < 6)
+                            weno_edges<false, false>(make_float2(a0[0], a1[0]), make_float2(a0[1], a1[1]), make_float2(a0[2], a1[2]),
+                                              make_float2(a0[3], a1[3]), make_float2(a0[4], a1[4]), r, l);
                         else
                         {
-                            const int g = row ? ty - 2 : j + 1;   // 1: y faces above, 2: x faces right
-                            if (g == 1) { dir = 1; src = L::kFy + TY * kTX + tx; }
-                            else
-                            {
-                                if (tx >= TY) continue;
-                                dir = 0; src = L::kFx + tx * (kTX + 1) + kTX;
-                            }
+                            weno_edges<false, false>(a0[0], a0[1], a0[2], a0[3], a0[4], r.x, l.x);
+                            weno_edges<false, false>(a1[0], a1[1], a1[2], a1[3], a1[4], r.y, l.y);
                         }
-#ifdef MPCF_CHECK_BOUNDS
-                        if (!face_slot(src)) { oob = true; continue; }
-#endif
-                        // x: normal u, transverse v, w;  y: normal v, transverse u, w
-                        T* pl = sm + src;
-                        const int nq = 1 + dir, tq = 2 - dir;
-                        FaceState<T> S;
-                        S.rm  = pl[0];              S.rp  = pl[7 * L::kFP];
-                        S.nm  = pl[nq * L::kFP];    S.np  = pl[(7 + nq) * L::kFP];
-                        S.t1m = pl[tq * L::kFP];    S.t1p = pl[(7 + tq) * L::kFP];
-                        S.t2m = pl[3 * L::kFP];     S.t2p = pl[10 * L::kFP];
-                        S.pm  = pl[4 * L::kFP];     S.pp  = pl[11 * L::kFP];
-                        S.Gm  = pl[5 * L::kFP];     S.Gp  = pl[12 * L::kFP];
-                        S.Pm  = pl[6 * L::kFP];     S.Pp  = pl[13 * L::kFP];
-                        FaceOut<T> o;
-                        face_hllc<Pol>(S, dir, o);
+                        smTw[MPCF_IN(d0, L::kYOff, L::kPP) * 4 + off] = r.x;
+                        smTw[MPCF_IN(d1, L::kYOff, L::kPP) * 4 + off] = r.y;
+                    };
+#pragma unroll 1
+                    for (int q = ty; q < 7; q += TY)
+                        edge_pair(L::kCurOff + 2 * L::kCurW + tx + 3, L::kCurW, L::kYOff + tx,
+                                  L::kCurOff + (TY + 3) * L::kCurW + tx + 3, -L::kCurW, L::kTopOff + tx, q);
+                    if (tx < TY)
+#pragma unroll 1
+                        for (int q = TY - 1 - ty; q < 7; q += TY)
+                            edge_pair(L::kCurOff + (tx + 3) * L::kCurW + 2, 1, L::kXgOff + tx,
+                                      L::kCurOff + (tx + 3) * L::kCurW + kTX + 3, -1, L::kXlOff + tx, q);
+                }
+                else
+                {
+                    // 21 jobs (3 of ghost_job x 7 quantities) in contiguous
+                    // ranges over the warps
+                    constexpr int kPer = 21 / TY, kRem = 21 % TY;
+                    int gi = ty * kPer + (ty < kRem ? ty : kRem);
+                    const int ge = gi + kPer + (ty < kRem ? 1 : 0);
+#pragma unroll 1
+                    for (; gi < ge; ++gi)
+                    {
+                        const int g = gi >= 14 ? 2 : (gi >= 7 ? 1 : 0);
+                        const int q = gi - 7 * g;
+                        int base, step, dst;
+                        if (!ghost_job<L, TY>(g, tx, base, step, dst)) continue;
+                        const int off = q % L::kPer + q / L::kPer * (L::kPP * L::kPer);
+                        // the reference's two edges are not mirror images bit
+                        // for bit: those forms take the cells left to right
+                        const int st = Pol::kFastWeno ? step : (step < 0 ? -step : step);
+                        T y[5], rv, lv;
 #pragma unroll
-                        for (int m = 0; m < 7; ++m) pl[m * L::kFP] = o.f[m];
-                        pl[7 * L::kFP] = o.Gm;  pl[8 * L::kFP] = o.Gp;
-                        pl[9 * L::kFP] = o.Pm;  pl[10 * L::kFP] = o.Pp;
-                        pl[11 * L::kFP] = o.vel;
+                        for (int i = 0; i < 5; ++i) y[i] = smT[MPCF_IN(base + (i - 2) * st, L::kCurOff, L::kYOff) * L::kPer + off];
+                        if constexpr (Pol::kFastWeno)
+                        {
+                            // (a mirrored stencil's left edge is its right edge)
+                            if (!weno_edges<false, true>(y[0], y[1], y[2], y[3], y[4], rv, lv))
+                                rv = weno_cell_call<Pol>(y[0], y[1], y[2], y[3], y[4]).R;
+                            lv = rv;
+                        }
+                        else                          weno_cell<Pol>(y[0], y[1], y[2], y[3], y[4], rv, lv);
+                        smTw[MPCF_IN(dst, L::kYOff, L::kPP) * L::kPer + off] = step > 0 ? rv : lv;
+                    }
+                }
+                __syncthreads();
+
+                // the register and state of plane k, for phase I of slab k+1
+                // (plane k-1's were last read before the barrier)
+                if (use_tma && threadIdx.x == 0 && !tma_late)
+                {
+                    fence_proxy_async();
+                    mbar_expect_tx(barC, 2 * (uint32_t)L::kBBytes);
+                    tma_load_4d(smem_u32(stC), tmR, x0, y0, k - DD.zlo, 0, barC);
+                    tma_load_4d(smem_u32(stC + 7 * L::kRing), tm + 128, x0, y0, k, 0, barC);
+                    pendC = true;
+                    parC = phC;
+                }
+                // ---- phase II: the y face below and the x face left of the
+                // own cell; the last two warps also the y faces above the
+                // tile and the x faces right of it
+                if constexpr (kPairFaces)
+                {
+                    T my[8], mx[8];
+                    ld8<T, L::kPP>(sm, L::kYOff + own, my);
+#pragma unroll
+                    for (int q = 0; q < 7; ++q) mx[q] = __shfl_up_sync(0xffffffffu, Rx[q], 1);
+                    mx[7] = (T)0;
+                    if (tx == 0) ld8<T, L::kPP>(sm, L::kXgOff + ty, mx);
+                    face_hllc_yx(my, Ly, mx, Lx, Fy, Fx);
+                    if (ty > 0) st8<T, L::kPP>(sm, L::kYOff + own, Fy);
+                }
+                constexpr int kFaceUnroll = Pol::kFastWeno ? 3 : 1;
+#pragma unroll kFaceUnroll
+                for (int j = kPairFaces ? 2 : 0; j < 3; ++j)
+                {
+                    if (j == 2 && ty < TY - 2) break;
+                    T m[8], p[8], f[8];
+                    int dir, dst = -1;
+                    if (j == 0)
+                    {
+                        ld8<T, L::kPP>(sm, L::kYOff + own, m);
+                        if constexpr (kStashLy) ld8<T, L::kPP>(sm, ring(r2), p);
+                        else
+                        {
+#pragma unroll
+                            for (int q = 0; q < 8; ++q) p[q] = Ly[q];
+                        }
+                        dir = 1;
+                        if (ty > 0) dst = L::kYOff + own;
+                    }
+                    else if (j == 1)
+                    {
+#pragma unroll
+                        for (int q = 0; q < 7; ++q) { m[q] = __shfl_up_sync(0xffffffffu, Rx[q], 1); p[q] = Lx[q]; }
+                        m[7] = p[7] = (T)0;
+                        if (tx == 0) ld8<T, L::kPP>(sm, L::kXgOff + ty, m);
+                        dir = 0;
+                    }
+                    else if (ty == TY - 1)
+                    {
+                        dst = L::kYOff + TY * kTX + tx;
+                        ld8<T, L::kPP>(sm, dst, m);
+                        ld8<T, L::kPP>(sm, L::kTopOff + tx, p);
+                        dir = 1;
+                    }
+                    else
+                    {
+                        if (tx >= TY) continue;
+                        dst = L::kXrOff + tx;
+                        ld8<T, L::kPP>(sm, dst, m);
+                        ld8<T, L::kPP>(sm, L::kXlOff + tx, p);
+                        dir = 0;
+                    }
+                    face_hllc<Pol>(m, p, dir, f);
+                    if (j == 0)
+                    {
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) Fy[q] = f[q];
+                    }
+                    if (j == 1)
+                    {
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) Fx[q] = f[q];
+                    }
+                    if (dst >= 0) st8<T, L::kPP>(sm, MPCF_IN(dst, L::kYOff, L::kPP), f);
+                }
+            }
+
+            // slab k+3 of the own column
+            {
+                T q[8];
+                if (use_tma)
+                {
+                    wait_copy(1);
+                    phB ^= 1;
+                    bool fx = false, fy = false, fz;
+                    int mx = tx, my = ty;
+                    if (!full)
+                    {
+                        mx = min(max(bc_map(gx, D.nx, D.bc0, D.bc1, fx) - x0, 0), kTX - 1);
+                        my = min(max(bc_map(gy, D.ny, D.bc2, D.bc3, fy) - y0, 0), TY - 1);
+                    }
+                    bc_map(k + 3, D.nz, D.bc4, D.bc5, fz);
+                    T c[7];
+                    const int bi = MPCF_IN(my * kTX + mx, 0, TY * kTX);
+#pragma unroll
+                    for (int m = 0; m < 7; ++m) c[m] = stB[m * TY * kTX + bi];
+                    if (fx) c[1] = -c[1];
+                    if (fy) c[2] = -c[2];
+                    if (fz) c[3] = -c[3];
+                    to_primitive<Pol>(c, q);
+                }
+                else load_prim<Pol>(D, U, gx, gy, k + 3, q, oob);
+                q[7] = (T)0;
+                st8<T, L::kPP>(sm, ring(r2), q);   // in place of slab k-2
+            }
+            // slab k+1 with halos into cur (k+1 < z1: no z mapping)
+            if (k + 1 < z1)
+            {
+                const bool box = use_tma && !full;
+                kcur = k + 1;
+                if (!box)
+                {
+                    // interior from the ring
+                    T q[8];
+                    ld8<T, L::kPP>(sm, ring(r2 + 3), q);
+                    st8<T, L::kPP>(sm, MPCF_IN(L::kCurOff + (ty + 3) * L::kCurW + tx + 3, L::kCurOff, L::kYOff), q);
+                }
+                if (use_tma)
+                {
+                    wait_copy(0);
+                    phA ^= 1;
+                }
+                // the 6*32 + 6*TY halo cells the x/y stencils read (the
+                // corners are never read); a tile reaching past the domain
+                // converts the whole staged box, its out-of-domain cells
+                // mapped to their sources
+                constexpr int kHalo = 6 * kTX + 6 * TY;
+                if (box)
+                {
+                    for (int i = threadIdx.x; i < (TY + 6) * L::kCurW; i += stage_threads<TY>())
+                    {
+                        const int ly = i / L::kCurW - 3, lx = i % L::kCurW - 3;
+                        convert_halo(halo_cell(lx, ly, true));
+                    }
+                }
+                else
+                {
+                    if (threadIdx.x < kHalo) convert_or_load(hc0, threadIdx.x);
+                    for (int i = threadIdx.x + stage_threads<TY>(); i < kHalo; i += stage_threads<TY>())
+                    {
+                        int lx, ly;
+                        halo_place(i, lx, ly);
+                        convert_or_load(halo_cell(lx, ly, !inner), i);
                     }
                 }
             }
+            r2 = r2 < 4 ? r2 + 1 : 0;
             __syncthreads();
-
-            // (F) x/y part of cell k, carried to the next slab
-            if (k < z1 && row)
-            {
-                // the slot right of / above the cell is read too
-                const T* fx = sm + L::kFx + MPCF_IN(ty * (kTX + 1) + tx, 0, L::kFP - 1);
-                const T* fy = sm + L::kFy + MPCF_IN(ty * kTX + tx, 0, L::kFP - kTX);
-#pragma unroll
-                for (int m = 0; m < 7; ++m)
-                    Sp[m] = ((fx[m * L::kFP + 1] - fx[m * L::kFP]) + fy[m * L::kFP + kTX]) - fy[m * L::kFP];
-                sG = fx[8 * L::kFP] + fx[7 * L::kFP + 1];
-                sP = fx[10 * L::kFP] + fx[9 * L::kFP + 1];
-                dU = fx[11 * L::kFP + 1] - fx[11 * L::kFP];
-                sG = sG + (fy[8 * L::kFP] + fy[7 * L::kFP + kTX]);
-                sP = sP + (fy[10 * L::kFP] + fy[9 * L::kFP + kTX]);
-                dU = dU + (fy[11 * L::kFP + kTX] - fy[11 * L::kFP]);
-            }
         }
 
         // ---- fused sound-speed maximum of the tile into its domain's
@@ -827,8 +979,7 @@ stage_kernel(const StageArgs A)
             __syncthreads();
             if (threadIdx.x < 32)
             {
-                // every warp of the CTA wrote its slot (a helper warp its 0)
-                T mm = threadIdx.x < TileShape<TY>::kWarps ? sos_w[threadIdx.x] : (T)0;
+                T mm = threadIdx.x < TY ? sos_w[threadIdx.x] : (T)0;
                 mm = shfl_max(mm);
                 if (threadIdx.x == 0) atomic_max_bits((char*)A.sos_bits + (size_t)d * sizeof(T), bad ? (T)NAN : mm);
             }
@@ -843,7 +994,7 @@ stage_kernel(const StageArgs A)
                 double v = cs[m];
 #pragma unroll
                 for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-                if (tx == 0 && row) red[ty * 5 + m] = v;
+                if (tx == 0) red[ty * 5 + m] = v;
             }
             __syncthreads();
             if (threadIdx.x < 5)
@@ -858,17 +1009,18 @@ stage_kernel(const StageArgs A)
         // after a wait ran out): wait for them, bounded, so that none lands
         // in shared memory the CTA no longer owns; a CTA that gave up takes
         // no further tile
-        if (TMA && threadIdx.x == 0 && (pendA || pendB))
+        if (TMA && threadIdx.x == 0 && (pendA || pendB || pendC))
         {
             if (pendA && !mbar_wait(barA, parA)) tma_inflight = true;
             if (pendB && !mbar_wait(barB, parB)) tma_inflight = true;
-            pendA = pendB = false;
+            if (pendC && !mbar_wait(barC, parC)) tma_inflight = true;
+            pendA = pendB = pendC = false;
         }
         if (!PERSIST) break;
         __syncthreads();
         if (threadIdx.x == 0) *tile_bc = tma_late ? A.ntiles : A.tile0 + (int)atomicAdd(A.counter, 1u);
         __syncthreads();
-        t = *tile_bc;
+        t = __shfl_sync(0xffffffffu, *tile_bc, 0);
     }
 
     if (!__all_sync(0xffffffffu, ok) && tx == 0) atomicOr(A.err, (unsigned)ERRBIT_NONPHYSICAL);

@@ -70,7 +70,7 @@ struct StageArgs
     unsigned* counter;  // persistent-launch work counter (zeroed before launch)
     unsigned* err;      // device error word
     double* tile_sums;  // [ntiles][5] FP64 partial conservation sums, or null
-    const void* tmaps;  // per domain 4 CUtensorMap (128 B each): [buffer 0, 1] x [halo box, interior box]
+    const void* tmaps;  // per domain 5 CUtensorMap (128 B each): [buffer 0, 1] x [halo box, interior box], register
     void* sos_bits;     // per domain maximum sound speed of the new state (bits), or null
     unsigned test_flags; // TEST_* below; 0 outside the failure-detection tests
 };

@@ -444,11 +444,11 @@ int mpcf_get_time(mpcf_solver* s, int dom, double* t);
 
 /* ---- launch configuration ------------------------------------------------- *
  * tile = 32 x ty columns x dz slabs (ty 3, 7 or 8; 15 also for
- * MPCF_PREC_FP32_REF), one CTA per tile of 32*(ty+1) threads for ty = 3, 7,
- * 15 (a helper warp evaluates the tile's extra faces) and 32*ty for ty = 8;
+ * MPCF_PREC_FP32_REF), one CTA of 32*ty threads per tile;
  * flags = MPCF_TILE_PERSISTENT | MPCF_TILE_TMA.  With MPCF_TILE_TMA, domains
  * whose rows are multiples of 16 bytes stage their slabs with bulk tensor
- * copies (other domains keep ordinary loads).  mpcf_autotune times the
+ * copies (other domains keep ordinary loads).  A new solver starts with
+ * 32 x 8 tiles and a depth chosen from its sizes.  mpcf_autotune times the
  * candidates on the solver's own state (which it leaves unchanged) and
  * keeps the fastest; best3 (optional) = {ty, dz, flags}, best_ms (optional)
  * = stage time. */
@@ -480,8 +480,9 @@ int mpcf_autotune(mpcf_solver* s, int reps, int* best3, double* best_ms);
 #define MPCF_TEST_DROP_LAST_COPY 1u
 #define MPCF_TEST_DROP_MID_COPY  2u
 int mpcf_set_test_flags(mpcf_solver* s, unsigned flags);
-/* Failure-detection tests only: bulk copies the stage kernel issued while a
- * test flag was set (clear != 0 resets the count).  No reference
+/* Failure-detection tests only: bulk copies of slabs (halo boxes and
+ * interiors ahead of the march) the stage kernel issued while a test flag
+ * was set (clear != 0 resets the count).  No reference
  * counterpart. */
 int mpcf_test_copy_count(mpcf_solver* s, unsigned* count, int clear);
 

@@ -1,0 +1,92 @@
+"""The stage kernel where its tiles, its fluxes' upwind choice and its
+branch-free weights can go wrong."""
+import numpy as np
+import pytest
+
+import oracle_lib as O
+from conftest import cloud_state
+from test_gpu_parity import assert_bitwise, rel_linf
+
+pytestmark = pytest.mark.gpu
+
+ABS, REF = 0, 1
+
+
+@pytest.mark.parametrize("dims", [(5, 5, 3), (32, 8, 1 + 2), (33, 9, 4), (64, 8, 8), (36, 7, 23), (65, 17, 19)])
+def test_default_tiling_matches_oracle(mpcf, dims):
+    """A new solver's tiling (its chunk depth follows the sizes; last chunks
+    and tiles are ragged) and depths 1 and 2: one step, bit for bit."""
+    bc = (REF, ABS, ABS, REF, REF, ABS)
+    U = cloud_state(dims, nb=1)
+    R = [np.zeros_like(a) for a in U]
+    U0 = [a.copy() for a in U]
+    dt_o, _ = O.step(dims, bc, U, R, cfl=0.3)
+    for dz in (None, 1, 2):
+        for persistent in (False, True):
+            with mpcf.Solver([dims], bc=[bc], precision="fp32_ref") as s:
+                if dz is not None:
+                    s.set_tiling(8, dz, persistent, True)
+                s.set_state(U0)
+                assert s.step(cfl=0.3)[0] == dt_o
+                Ug, Rg = s.get_state()
+                assert s.error_word() == 0
+            assert_bitwise(Ug, U, f"state, dz {dz}")
+            assert_bitwise(Rg, R, f"register, dz {dz}")
+
+
+def test_contact_at_rest_and_nan_velocity(mpcf):
+    """s* = 0 on every face (uniform pressure, no velocity, a density jump):
+    both sides' fluxes are blended, as in the reference.  A NaN transverse
+    momentum in one cell reaches the same cells as in the reference's
+    two-sided sum."""
+    dims = (40, 16, 12)
+    n = dims[0] * dims[1] * dims[2]
+    x = np.arange(n) % dims[0]
+    rho = np.where(x < 17, 1000.0, 1.0).astype(np.float32)
+    zero = np.zeros(n, np.float32)
+    G = np.full(n, 2.5, np.float32)
+    E = np.full(n, 250.0, np.float32)
+    for nan in (False, True):
+        v = zero.copy()
+        if nan:
+            v[:] = 3.0 * rho                       # s* != 0 in y: upwind fluxes
+            v[20 + dims[0] * (7 + dims[1] * 5)] = np.nan
+        U = [rho.copy(), (2.0 * rho if nan else zero).copy(), v, zero.copy(), E + 20 * rho, G.copy(), zero.copy()]
+        U = [np.ascontiguousarray(a, np.float32) for a in U]
+        R = [np.zeros_like(a) for a in U]
+        U0 = [a.copy() for a in U]
+        O.stage(dims, (ABS,) * 6, U, R, 0.0, 0.25, 0.01)
+        with mpcf.Solver([dims], precision="fp32_ref") as s:
+            s.set_state(U0)
+            s.stage(0.0, 0.25, 0.01)
+            Ug, Rg = s.get_state()
+        assert_bitwise(Ug, U, f"state, nan {nan}")
+        assert_bitwise(Rg, R, f"register, nan {nan}")
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp64_fast"])
+@pytest.mark.parametrize("scale", [1.0, 1e16, 1e22, 1e60])
+def test_fp64_weights_over_the_range_of_scales(mpcf, prec, scale):
+    """Pressures from 1 to 1e60: above about 1e18 the fast form's shared
+    reciprocal leaves its range (1e22) and above 1e75 the reference form's
+    products would; both then take their general forms.  Random cells, so
+    the indicators do not cancel; one stage against the FP64 oracle, whose
+    1/6 of the extra terms is the reference's float literal, 5e-9 off: with
+    dt/h divU of order 0.1 that moves G by less than 1e-8 (all else differs
+    by contraction, 2^-53 times a few hundred operations)."""
+    dims = (34, 18, 9)
+    rng = np.random.default_rng(5)
+    n = dims[0] * dims[1] * dims[2]
+    p = scale * rng.uniform(0.5, 2.0, n)
+    U = [rng.uniform(1.0, 2.0, n), np.zeros(n), np.zeros(n), np.zeros(n), 2.5 * p, np.full(n, 2.5), np.zeros(n)]
+    R = [np.zeros(n) for _ in range(7)]
+    U0 = [a.copy() for a in U]
+    dtinvh = 0.1 / np.sqrt(1.4 * 2 * scale)
+    O.stage(dims, (ABS,) * 6, U, R, 0.0, 0.25, dtinvh)
+    with mpcf.Solver([dims], precision=prec) as s:
+        s.set_state(U0)
+        s.stage(0.0, 0.25, dtinvh)
+        Ug, _ = s.get_state()
+    for q in range(7):
+        assert np.isfinite(Ug[q]).all()
+        assert rel_linf(Ug[q], U[q]) <= 1e-8, (q, rel_linf(Ug[q], U[q]))
