@@ -119,6 +119,7 @@ struct mpcf_solver
 
     // launch configuration
     int ty = 7, dz = 64, persist = 0, tma = 0;
+    bool tma_all = false;           // every domain qualifies for bulk copies
     int ntiles = 0;
     int sos_chunk = 32768, nchunks = 0;
     bool track_cons = false;
@@ -178,16 +179,18 @@ StageKernelInfo stage_info(const mpcf_solver* s, int ty, bool persist, bool sums
 
 cudaError_t launch_stage(const mpcf_solver* s, const StageArgs& A, int grid, cudaStream_t st)
 {
+    // the bulk-copy instance takes domains that all qualify
+    const bool tma = s->tma && s->tma_all;
     if (s->weno3)
-        return s->pol == 0 ? launch_stage_ref_w3(s->ty, s->persist != 0, s->tma != 0, A, grid, st)
-                           : launch_stage_fp64_w3(s->ty, s->persist != 0, s->tma != 0, A, grid, st);
+        return s->pol == 0 ? launch_stage_ref_w3(s->ty, s->persist != 0, tma, A, grid, st)
+                           : launch_stage_fp64_w3(s->ty, s->persist != 0, tma, A, grid, st);
     switch (s->pol)
     {
-        case 0: return launch_stage_ref(s->ty, s->persist != 0, s->tma != 0, A, grid, st);
-        case 1: return launch_stage_fast32(s->ty, s->persist != 0, s->tma != 0, A, grid, st);
-        case 2: return launch_stage_mixed(s->ty, s->persist != 0, s->tma != 0, A, grid, st);
-        case 4: return launch_stage_fast64(s->ty, s->persist != 0, s->tma != 0, A, grid, st);
-        default: return launch_stage_fp64(s->ty, s->persist != 0, s->tma != 0, A, grid, st);
+        case 0: return launch_stage_ref(s->ty, s->persist != 0, tma, A, grid, st);
+        case 1: return launch_stage_fast32(s->ty, s->persist != 0, tma, A, grid, st);
+        case 2: return launch_stage_mixed(s->ty, s->persist != 0, tma, A, grid, st);
+        case 4: return launch_stage_fast64(s->ty, s->persist != 0, tma, A, grid, st);
+        default: return launch_stage_fp64(s->ty, s->persist != 0, tma, A, grid, st);
     }
 }
 
@@ -309,6 +312,8 @@ int apply_tiling(mpcf_solver* s)
         if ((rc = dev_alloc(s, (void**)&s->chunk_sums, sizeof(double) * 5 * (size_t)std::max(c, 1)))) return rc;
     if ((rc = encode_tensor_maps(s))) return rc;
     if (s->tma && !any_tma_ok(s)) s->tma = 0;
+    s->tma_all = true;
+    for (const auto& D : s->hdoms) s->tma_all = s->tma_all && D.tma_ok;
     CK(cudaMemcpyAsync(s->ddoms, s->hdoms.data(), sizeof(DomDev) * s->ndom, cudaMemcpyHostToDevice, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     destroy_graphs(s);

@@ -37,17 +37,21 @@
 // ping-ponged (read U[parity], write U[parity^1]) so neighbouring tiles
 // always see the old state.
 //
-// Loads.  Without TMA every thread loads its cells with ordinary global
-// loads (the generic path, any domain shape).  With TMA (domains whose rows
-// are multiples of 16 bytes), one elected thread issues four bulk tensor
-// copies per slab into shared memory: in phase I the 40 x (TY+6) halo box of
-// the next slab and the 32 x TY interior of the slab three ahead, which phase
-// II converts (out-of-domain cells of the staged box are mapped to their
-// mirror / clamp source inside the box); in phase II the register and the
-// state of the plane that the next phase I finalises.  Waits on the copies
-// are bounded: a copy that does not complete sets an error bit, the CTA stops
-// waiting for copies and carries on (its data are then stale, never out of
-// bounds), so a failed copy cannot stall the launch.
+// Loads.  With TMA (solvers whose domains' rows are all multiples of 16
+// bytes), three staging buffers in shared memory are filled while a phase is
+// worked on, by four bulk tensor copies per slab that one elected thread
+// issues: in phase I the halo of the next slab (a 40 x (TY+6) box, whose
+// out-of-domain cells are mapped to their mirror / clamp source inside the
+// box) and the interior of the slab three ahead, which phase II converts; in
+// phase II the register and the state of the plane that the next phase I
+// finalises.  Waits on the copies are bounded: a copy that does not complete
+// sets an error bit, the CTA stops waiting for copies and carries on (its
+// data are then stale, never out of bounds), so a failed copy cannot stall
+// the launch.  Otherwise (any domain shape) every thread loads its cells with
+// ordinary loads (per-thread cp.async into the staging buffers was 10-19 %
+// slower on rows that are no multiples of 16 bytes, prefetching the slabs
+// ahead into L1 2 %).  An instance has one of the two: with both, each was
+// 2-4 % slower.
 //
 // DRAM traffic per cell-stage: read U (7 T) + read R (7 T) + write R and
 // U_next (14 T) = 112 B in FP32.  Halo and ring re-reads hit L2.
@@ -337,7 +341,7 @@ __device__ __forceinline__ void weno_record(const typename Vec16<typename Pol::T
                 else                          ok &= weno_cell_ref<Pol, true>(y[0][i], y[1][i], y[2][i], y[3][i], y[4][i], R[q], L[q]);
                 // two quantities at a time: more overlap than this spills
                 // (fast form, 256^3: 11.5 ms a step, 13.1 without the fences)
-                if (q % 2 == (Pol::kFastWeno ? 0 : 1)) __syncwarp();
+                if (q % 2 == 0) __syncwarp();
             }
             else
                 weno_cell<Pol>(y[0][i], y[1][i], y[2][i], y[3][i], y[4][i], R[q], L[q]);
@@ -474,7 +478,7 @@ stage_kernel(const StageArgs A)
         T* __restrict__       Un   = (T*)DD.Ux[A.parity ^ 1];
         T* __restrict__       R    = (T*)DD.Rx;
         const T dtinvh = ((const T*)A.dtinvh)[d];
-        const bool use_tma = TMA && DD.tma_ok;
+        constexpr bool use_tma = TMA;
         // tensor maps of the buffer read in this stage (halo box, interior
         // box) and of the register (interior box, own planes only)
         const char* tm = (const char*)A.tmaps + ((size_t)d * 5 + (size_t)A.parity * 2) * 128;
@@ -514,6 +518,70 @@ stage_kernel(const StageArgs A)
             else      issue(tm, false, x0, y0, bc_map(k + 3, D.nz, D.bc4, D.bc5, fz));
             if (k + 1 < z1) issue(tm, true, x0 - 4, y0 - 3, bc_map(k + 1, D.nz, D.bc4, D.bc5, fz));
         };
+        // halo cell i (0 .. 6*32 + 6*TY - 1: the cells the x/y stencils read;
+        // the corners are never read) at (lx, ly) relative to the tile
+        auto halo_place = [&](const int i, int& lx, int& ly)
+        {
+            if (i < 6 * kTX) { const int r = i >> 5; lx = i & (kTX - 1); ly = r < 3 ? r - 3 : TY + r - 3; }
+            else             { const int j = i - 6 * kTX, c = j % 6; ly = j / 6; lx = c < 3 ? c - 3 : kTX + c - 3; }
+        };
+        // its cell of the staged box (a bulk copy's box holds the domain's own
+        // cells), its record in cur and the momenta its boundary condition
+        // flips, packed: box | cur << 12 | fx << 30 | fy << 31
+        auto halo_cell = [&](const int lx, const int ly, const bool map)
+        {
+            bool fx = false, fy = false;
+            int mx = lx + 4, my = ly + 3;
+            if (map)
+            {
+                const int sx = bc_map(x0 + lx, D.nx, D.bc0, D.bc1, fx), sy = bc_map(y0 + ly, D.ny, D.bc2, D.bc3, fy);
+                if (use_tma)
+                {
+                    mx = min(max(sx - x0 + 4, 0), L::kAW - 1);
+                    my = min(max(sy - y0 + 3, 0), L::kAH - 1);
+                }
+            }
+            return (unsigned)(my * L::kAW + mx) | (unsigned)(L::kCurOff + (ly + 3) * L::kCurW + lx + 3) << 12 |
+                   (fx ? 1u << 30 : 0u) | (fy ? 1u << 31 : 0u);
+        };
+        auto convert_halo = [&](const unsigned hc, const int i, const int k)
+        {
+            T q[8];
+            if (use_tma)
+            {
+                T c[7];
+                const int ai = MPCF_IN((int)(hc & 0xfffu), 0, L::kAH * L::kAW);
+#pragma unroll
+                for (int m = 0; m < 7; ++m) c[m] = stA[m * L::kAH * L::kAW + ai];
+                if (hc >> 30 & 1u) c[1] = -c[1];
+                if (hc >> 31)      c[2] = -c[2];
+                to_primitive<Pol>(c, q);
+            }
+            else
+            {
+                int lx, ly;
+                halo_place(i, lx, ly);
+                load_prim<Pol>(D, U, x0 + lx, y0 + ly, k, q, oob);
+            }
+            q[7] = (T)0;
+            st8<T, L::kPP>(sm, MPCF_IN((int)(hc >> 12 & 0x3ffffu), L::kCurOff, L::kYOff), q);
+        };
+        int hlx, hly;
+        halo_place(threadIdx.x, hlx, hly);
+        const unsigned hc0 = halo_cell(hlx, hly, !inner);
+        // the own column's cell of a staged interior and the momenta its
+        // boundary condition flips
+        bool own_fx, own_fy;
+        const int own_sx = bc_map(gx, D.nx, D.bc0, D.bc1, own_fx), own_sy = bc_map(gy, D.ny, D.bc2, D.bc3, own_fy);
+        const int own_b = use_tma && !full ? min(max(own_sy - y0, 0), TY - 1) * kTX + min(max(own_sx - x0, 0), kTX - 1) : own;
+        // without bulk copies: lane l < 28 prefetches a row piece for the
+        // finalisation: field l % 7 of R / U, first / second line
+        const T* pf = U;
+        if (!use_tma)
+        {
+            const int f = tx % 7, w = tx / 7;
+            pf = ((w & 1) ? U : (const T*)R) + f * D.fs - (long long)D.nx * D.ny + (long long)D.nx * min(gy, D.ny - 1) + min(x0 + ((w & 2) ? 31 : 0), D.nx - 1);
+        }
         if (use_tma && threadIdx.x == 0 && !tma_late) issue_for(z0 - 1);
 
         // ---- prologue: slabs z0-3 .. z0+1 of the own column into the ring
@@ -526,53 +594,6 @@ stage_kernel(const StageArgs A)
             st8<T, L::kPP>(sm, ring(j), q);
         }
 
-        // halo cell i (0 .. 6*32 + 6*TY - 1: the cells the x/y stencils read;
-        // the corners are never read) at (lx, ly) relative to the tile
-        auto halo_place = [&](const int i, int& lx, int& ly)
-        {
-            if (i < 6 * kTX) { const int r = i >> 5; lx = i & (kTX - 1); ly = r < 3 ? r - 3 : TY + r - 3; }
-            else             { const int j = i - 6 * kTX, c = j % 6; ly = j / 6; lx = c < 3 ? c - 3 : kTX + c - 3; }
-        };
-        // its cell of the staged box, its record in cur and the momenta its
-        // boundary condition flips, packed: box | cur << 12 | fx << 30 | fy << 31
-        auto halo_cell = [&](const int lx, const int ly, const bool map)
-        {
-            bool fx = false, fy = false;
-            int mx = lx + 4, my = ly + 3;
-            if (map)
-            {
-                mx = min(max(bc_map(x0 + lx, D.nx, D.bc0, D.bc1, fx) - x0 + 4, 0), L::kAW - 1);
-                my = min(max(bc_map(y0 + ly, D.ny, D.bc2, D.bc3, fy) - y0 + 3, 0), L::kAH - 1);
-            }
-            return (unsigned)(my * L::kAW + mx) | (unsigned)(L::kCurOff + (ly + 3) * L::kCurW + lx + 3) << 12 |
-                   (fx ? 1u << 30 : 0u) | (fy ? 1u << 31 : 0u);
-        };
-        auto convert_halo = [&](const unsigned hc)
-        {
-            T c[7], q[8];
-            const int ai = MPCF_IN((int)(hc & 0xfffu), 0, L::kAH * L::kAW);
-#pragma unroll
-            for (int m = 0; m < 7; ++m) c[m] = stA[m * L::kAH * L::kAW + ai];
-            if (hc >> 30 & 1u) c[1] = -c[1];
-            if (hc >> 31)      c[2] = -c[2];
-            to_primitive<Pol>(c, q);
-            q[7] = (T)0;
-            st8<T, L::kPP>(sm, MPCF_IN((int)(hc >> 12 & 0x3ffffu), L::kCurOff, L::kYOff), q);
-        };
-        int hlx, hly;
-        halo_place(threadIdx.x, hlx, hly);
-        const unsigned hc0 = halo_cell(hlx, hly, !inner);
-        int kcur = 0;
-        auto convert_or_load = [&](const unsigned hc, const int i)
-        {
-            if (use_tma) { convert_halo(hc); return; }
-            int lx, ly;
-            halo_place(i, lx, ly);
-            T q[8];
-            load_prim<Pol>(D, U, x0 + lx, y0 + ly, kcur, q, oob);
-            q[7] = (T)0;
-            st8<T, L::kPP>(sm, MPCF_IN((int)(hc >> 12 & 0x3ffffu), L::kCurOff, L::kYOff), q);
-        };
         // carried from slab to slab: the z face below, the upper z edge and
         // the x/y faces left of / below the cell, the G/P sums of its edges
         T zfp[8], Rz[8], Fx[8], Fy[8];
@@ -583,12 +604,6 @@ stage_kernel(const StageArgs A)
         T smax = 0;              // fused sound speed of the new state (last stage)
         bool sbad = false;
 
-        // lane l < 28 prefetches row piece l: field l % 7 of R / U, first / second line
-        const T* pf;
-        {
-            const int f = tx % 7, w = tx / 7;
-            pf = ((w & 1) ? U : (const T*)R) + f * D.fs - (long long)D.nx * D.ny + (long long)D.nx * min(gy, D.ny - 1) + min(x0 + ((w & 2) ? 31 : 0), D.nx - 1);
-        }
         // slab z0-1 gives its upper z edge only
         int r2 = 0;
 #pragma unroll 1
@@ -597,11 +612,10 @@ stage_kernel(const StageArgs A)
             const bool xy = k >= z0 && k < z1;     // slab k has x and y faces
             // the staging buffers are free again (phase II of slab k-1 is
             // behind the barrier): copy while this slab is worked on
-            if (use_tma && threadIdx.x == 0 && !tma_late && xy) issue_for(k);
+            if (use_tma) { if (threadIdx.x == 0 && !tma_late && xy) issue_for(k); }
+            else if (k > z0 && tx < 28) prefetch_l1(pf + (long long)D.nx * D.ny * k);
 
             // ---- phase I
-            // without bulk copies, R and U of cell k-1 are first prefetched
-            // into L1, so that its finalisation after the z face finds them
             const bool fin = (k > z0) && valid;
 #ifdef MPCF_CHECK_BOUNDS
             // cell k-1 of the own column: inside the domain's own planes
@@ -611,7 +625,6 @@ stage_kernel(const StageArgs A)
 #else
             const long long idx = (long long)gx + (long long)D.nx * ((long long)gy + (long long)D.ny * (k - 1));
 #endif
-            if (!use_tma && k > z0 && tx < 28) prefetch_l1(pf + (long long)D.nx * D.ny * k);
             // x/y part of cell k-1: its own faces, the face right of it from
             // the next lane (or the tile's extra face) and the face above it
             // from its slot
@@ -655,15 +668,11 @@ stage_kernel(const StageArgs A)
                 if (fin)
                 {
                     T Rold[7], Uold[7];
-                    if (use_tma)
-                    {
 #pragma unroll
-                        for (int m = 0; m < 7; ++m) { Rold[m] = stC[m * L::kRing + own]; Uold[m] = stC[(7 + m) * L::kRing + own]; }
-                    }
-                    else
+                    for (int m = 0; m < 7; ++m)
                     {
-#pragma unroll
-                        for (int m = 0; m < 7; ++m) { Rold[m] = R[m * D.fs + idx]; Uold[m] = __ldg(U + m * D.fs + idx); }
+                        Rold[m] = use_tma ? stC[m * L::kRing + own] : R[m * D.fs + idx];
+                        Uold[m] = use_tma ? stC[(7 + m) * L::kRing + own] : __ldg(U + m * D.fs + idx);
                     }
                     const T divU = dU + (zf[7] - zfp[7]);
                     T un[7];
@@ -897,26 +906,19 @@ stage_kernel(const StageArgs A)
             }
 
             // slab k+3 of the own column
+            if (use_tma) { wait_copy(1); phB ^= 1; }
             {
                 T q[8];
                 if (use_tma)
                 {
-                    wait_copy(1);
-                    phB ^= 1;
-                    bool fx = false, fy = false, fz;
-                    int mx = tx, my = ty;
-                    if (!full)
-                    {
-                        mx = min(max(bc_map(gx, D.nx, D.bc0, D.bc1, fx) - x0, 0), kTX - 1);
-                        my = min(max(bc_map(gy, D.ny, D.bc2, D.bc3, fy) - y0, 0), TY - 1);
-                    }
+                    bool fz;
                     bc_map(k + 3, D.nz, D.bc4, D.bc5, fz);
                     T c[7];
-                    const int bi = MPCF_IN(my * kTX + mx, 0, TY * kTX);
+                    const int bi = MPCF_IN(own_b, 0, L::kRing);
 #pragma unroll
-                    for (int m = 0; m < 7; ++m) c[m] = stB[m * TY * kTX + bi];
-                    if (fx) c[1] = -c[1];
-                    if (fy) c[2] = -c[2];
+                    for (int m = 0; m < 7; ++m) c[m] = stB[m * L::kRing + bi];
+                    if (own_fx) c[1] = -c[1];
+                    if (own_fy) c[2] = -c[2];
                     if (fz) c[3] = -c[3];
                     to_primitive<Pol>(c, q);
                 }
@@ -928,7 +930,6 @@ stage_kernel(const StageArgs A)
             if (k + 1 < z1)
             {
                 const bool box = use_tma && !full;
-                kcur = k + 1;
                 if (!box)
                 {
                     // interior from the ring
@@ -951,17 +952,17 @@ stage_kernel(const StageArgs A)
                     for (int i = threadIdx.x; i < (TY + 6) * L::kCurW; i += stage_threads<TY>())
                     {
                         const int ly = i / L::kCurW - 3, lx = i % L::kCurW - 3;
-                        convert_halo(halo_cell(lx, ly, true));
+                        convert_halo(halo_cell(lx, ly, true), 0, k + 1);
                     }
                 }
                 else
                 {
-                    if (threadIdx.x < kHalo) convert_or_load(hc0, threadIdx.x);
+                    if (threadIdx.x < kHalo) convert_halo(hc0, threadIdx.x, k + 1);
                     for (int i = threadIdx.x + stage_threads<TY>(); i < kHalo; i += stage_threads<TY>())
                     {
                         int lx, ly;
                         halo_place(i, lx, ly);
-                        convert_or_load(halo_cell(lx, ly, !inner), i);
+                        convert_halo(halo_cell(lx, ly, !inner), i, k + 1);
                     }
                 }
             }
