@@ -141,6 +141,10 @@ struct mpcf_solver
     // per-chunk events, made on first use
     cudaStream_t up = nullptr, down = nullptr;
     std::vector<cudaEvent_t> ev_up, ev_st, ev_down;
+    // streamed and windowed runs: streams of stages 2 and 3 (stage 1: the
+    // solver's) and the events of stages 1 and 2 per chunk
+    cudaStream_t st23[2] = {nullptr, nullptr};
+    std::vector<cudaEvent_t> ev_k[2];
     cudaEvent_t ev_start = nullptr;
 
     // windowed runs (mpcf_create_window / mpcf_run_window): the domains are
@@ -459,22 +463,26 @@ StageArgs stage_args(mpcf_solver* s, double a, double b, bool sums)
     return A;
 }
 
-// Enqueue the stage of tiles [tile_lo, tile_hi) on the solver's stream
-// (device dt/h); the parity is left as it is (the caller flips it once the
-// whole stage is enqueued).
-int enqueue_stage_tiles(mpcf_solver* s, double a, double b, bool sums, bool sos, int tile_lo, int tile_hi)
+// Enqueue the stage of tiles [tile_lo, tile_hi) on the solver's stream, or
+// on stream `st` with the work counter of `lane` (launches that may overlap
+// have different lanes), with the device dt/h; the parity is left as it is
+// (the caller flips it once the whole stage is enqueued).
+int enqueue_stage_tiles(mpcf_solver* s, double a, double b, bool sums, bool sos, int tile_lo, int tile_hi,
+                        cudaStream_t st = nullptr, int lane = 0)
 {
+    if (!st) st = s->stream;
     StageArgs A = stage_args(s, a, b, sums);
     if (sos) A.sos_bits = s->sos_bits;
+    A.counter = s->counter + (lane ? lane + 1 : 0);     // (1 counts copies in failure-detection tests)
     A.tile0 = tile_lo;
     A.ntiles = tile_hi;
     int grid = tile_hi - tile_lo;
     if (s->persist)
     {
         grid = std::min(grid, persistent_grid(s, s->ty));
-        CK(cudaMemsetAsync(s->counter, 0, sizeof(unsigned), s->stream));
+        CK(cudaMemsetAsync(A.counter, 0, sizeof(unsigned), st));
     }
-    cudaError_t e = launch_stage(s, A, grid, s->stream);
+    cudaError_t e = launch_stage(s, A, grid, st);
     if (e != cudaSuccess) return fail(MPCF_ERR_CUDA, "stage launch failed: %s", cudaGetErrorString(e));
     return MPCF_OK;
 }
@@ -541,6 +549,24 @@ int enqueue_step(mpcf_solver* s, double cfl, double dt_max, bool standalone_sos)
     if ((rc = enqueue_dt(s, cfl, dt_max))) return rc;
     for (int k = 0; k < 3; ++k)
         if ((rc = enqueue_stage(s, kLSRK3[k][0], kLSRK3[k][1], s->track_cons && k == 2, k == 2))) return rc;
+    return MPCF_OK;
+}
+
+// Streams of the streamed and windowed runs, made on first use: two for the
+// copies and one each for stages 2 and 3, later stages first (their results
+// are what the downloads, and then the next step's uploads, wait for).  A
+// launch over one chunk rarely fills the device's resident slots by whole
+// rounds; independent stages of other chunks fill the rest.
+int stream_setup(mpcf_solver* s)
+{
+    if (s->up) return MPCF_OK;
+    int lo = 0, hi = 0;
+    CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+    CK(cudaStreamCreateWithPriority(&s->st23[0], cudaStreamNonBlocking, std::max(hi, lo - 1)));
+    CK(cudaStreamCreateWithPriority(&s->st23[1], cudaStreamNonBlocking, hi));
+    CK(cudaEventCreateWithFlags(&s->ev_start, cudaEventDisableTiming));
+    CK(cudaStreamCreateWithFlags(&s->down, cudaStreamNonBlocking));
+    CK(cudaStreamCreateWithFlags(&s->up, cudaStreamNonBlocking));
     return MPCF_OK;
 }
 
@@ -700,9 +726,9 @@ int mpcf_destroy(mpcf_solver* s)
     if (!s) return MPCF_OK;
     DeviceGuard g(s->device);
     if (s->stream) cudaStreamSynchronize(s->stream);
-    for (cudaStream_t c : {s->up, s->down})
+    for (cudaStream_t c : {s->up, s->down, s->st23[0], s->st23[1]})
         if (c) { cudaStreamSynchronize(c); cudaStreamDestroy(c); }
-    for (auto* v : {&s->ev_up, &s->ev_st, &s->ev_down, &s->ev_free_c, &s->ev_free_d})
+    for (auto* v : {&s->ev_up, &s->ev_st, &s->ev_down, &s->ev_free_c, &s->ev_free_d, &s->ev_k[0], &s->ev_k[1]})
         for (cudaEvent_t e : *v) cudaEventDestroy(e);
     if (s->ev_start) cudaEventDestroy(s->ev_start);
     destroy_graphs(s);
@@ -961,13 +987,9 @@ int mpcf_run_host(mpcf_solver* s, int nsteps, double cfl, double dt_max, void* c
         zc[c] = std::min(D.nz, lc[c] * s->dz);
     }
     // streams and events, made once
-    if (!s->up)
-    {
-        CK(cudaStreamCreateWithFlags(&s->up, cudaStreamNonBlocking));
-        CK(cudaStreamCreateWithFlags(&s->down, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&s->ev_start, cudaEventDisableTiming));
-    }
-    for (auto* v : {&s->ev_up, &s->ev_st, &s->ev_down})
+    int rc;
+    if ((rc = stream_setup(s))) return rc;
+    for (auto* v : {&s->ev_up, &s->ev_st, &s->ev_down, &s->ev_k[0], &s->ev_k[1]})
         while ((int)v->size() < nch)
         {
             cudaEvent_t e;
@@ -988,7 +1010,7 @@ int mpcf_run_host(mpcf_solver* s, int nsteps, double cfl, double dt_max, void* c
     // queued on the solver's stream
     CK(cudaEventRecord(s->ev_start, s->stream));
     CK(cudaStreamWaitEvent(s->up, s->ev_start, 0));
-    int rc;
+    cudaStream_t str[3] = {s->stream, s->st23[0], s->st23[1]};
     for (int n = 0; n < nsteps; ++n)
     {
         const int p = s->parity;
@@ -1029,13 +1051,16 @@ int mpcf_run_host(mpcf_solver* s, int nsteps, double cfl, double dt_max, void* c
                 done = upto;
             }
         }
+        if (n > 0) CK(cudaStreamWaitEvent(s->stream, s->ev_st[nch - 1], 0));   // the last stage 3
         if ((rc = enqueue_dt(s, cfl, dt_max))) return rc;
-        // (3) the three stages as a wavefront over the chunks: stage k of
-        // chunk c follows stage k-1 (stage 1: the upload) of chunks
-        // 0..hi[c].  Stage k reads buffer p ^ (k & 1) and writes the other;
-        // a chunk's stage overwrites planes that only the previous stage of
-        // chunks up to hi[c] read, so these read-after-write orders also
-        // cover the buffers' reuse.  Stage 3 accumulates the sound speed of
+        // (3) the three stages as a wavefront over the chunks, each stage on
+        // its own stream: stage k of chunk c follows stage k-1 (stage 1: the
+        // upload) of chunks 0..hi[c].  Stage k reads buffer p ^ (k & 1) and
+        // writes the other; a chunk's stage overwrites planes that only the
+        // previous stage of chunks up to hi[c] read, so these
+        // read-after-write orders also cover the buffers' reuse.  (Stage k-1
+        // of a chunk above hi[c], which may run at the same time, reads no
+        // plane of chunk c.)  Stage 3 accumulates the sound speed of
         // the state it writes (the next step's dt) and hands each chunk to
         // the download stream.
         int d[3] = {0, 0, 0};
@@ -1045,12 +1070,12 @@ int mpcf_run_host(mpcf_solver* s, int nsteps, double cfl, double dt_max, void* c
             if (d[1] > hi[d[2]]) k = 2;
             else if (d[1] < nch && d[0] > hi[d[1]]) k = 1;
             const int c = d[k]++;
-            if (k == 0) CK(cudaStreamWaitEvent(s->stream, s->ev_up[hi[c]], 0));
+            CK(cudaStreamWaitEvent(str[k], k == 0 ? s->ev_up[hi[c]] : s->ev_k[k - 1][hi[c]], 0));
             s->parity = p ^ (k & 1);
-            rc = enqueue_stage_tiles(s, kLSRK3[k][0], kLSRK3[k][1], false, k == 2, lc[c] * txy, lc[c + 1] * txy);
+            rc = enqueue_stage_tiles(s, kLSRK3[k][0], kLSRK3[k][1], false, k == 2, lc[c] * txy, lc[c + 1] * txy, str[k], k);
             s->parity = p;
             if (rc) return rc;
-            if (k == 2) CK(cudaEventRecord(s->ev_st[c], s->stream));
+            CK(cudaEventRecord(k == 2 ? s->ev_st[c] : s->ev_k[k][c], str[k]));
         }
         s->parity = p ^ 1;
         const char* res = (const char*)D.U[p ^ 1];
@@ -1068,8 +1093,7 @@ int mpcf_run_host(mpcf_solver* s, int nsteps, double cfl, double dt_max, void* c
     // accumulator holds its maximum (from the last stage 3)
     if (nsteps > 0) s->sos_fresh = true;
     s->sums_valid = false;
-    CK(cudaStreamSynchronize(s->down));
-    CK(cudaStreamSynchronize(s->up));
+    for (cudaStream_t c : {s->down, s->up, str[1], str[2]}) CK(cudaStreamSynchronize(c));
     if (time_out) CK(cudaMemcpyAsync(time_out, s->time, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     return MPCF_OK;
@@ -1221,12 +1245,8 @@ bool window_stage_plan(const int nch, const int ns, std::vector<WinOp>& plan)
 int window_begin(mpcf_solver* s)
 {
     const int nch = s->win_nch, ns = s->ndom;
-    if (!s->up)
-    {
-        CK(cudaStreamCreateWithFlags(&s->up, cudaStreamNonBlocking));
-        CK(cudaStreamCreateWithFlags(&s->down, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&s->ev_start, cudaEventDisableTiming));
-    }
+    int rc = stream_setup(s);
+    if (rc) return rc;
     auto grow = [&](std::vector<cudaEvent_t>& v, const int n)
     {
         while ((int)v.size() < n)
@@ -1237,7 +1257,8 @@ int window_begin(mpcf_solver* s)
         }
         return true;
     };
-    if (!grow(s->ev_up, nch) || !grow(s->ev_st, nch) || !grow(s->ev_free_c, ns) || !grow(s->ev_free_d, ns))
+    if (!grow(s->ev_up, nch) || !grow(s->ev_st, nch) || !grow(s->ev_k[0], nch) || !grow(s->ev_k[1], nch) ||
+        !grow(s->ev_free_c, ns) || !grow(s->ev_free_d, ns))
     { cudaGetLastError(); return fail(MPCF_ERR_CUDA, "cudaEventCreate failed"); }
     CK(cudaEventRecord(s->ev_start, s->stream));
     CK(cudaStreamWaitEvent(s->up, s->ev_start, 0));
@@ -1254,9 +1275,7 @@ int window_end(mpcf_solver* s)
 {
     s->sos_fresh = false;
     s->sums_valid = false;
-    CK(cudaStreamSynchronize(s->down));
-    CK(cudaStreamSynchronize(s->up));
-    CK(cudaStreamSynchronize(s->stream));
+    for (cudaStream_t c : {s->down, s->up, s->st23[0], s->st23[1], s->stream}) CK(cudaStreamSynchronize(c));
     return MPCF_OK;
 }
 
@@ -1385,6 +1404,7 @@ int mpcf_run_window(mpcf_solver* s, int nsteps, double cfl, double dt_max, void*
     if ((rc = window_begin(s))) return rc;
     CK(cudaMemsetAsync(s->sos_bits, 0, esz * ns, s->stream));
     const int p0 = s->parity;
+    cudaStream_t str[3] = {s->stream, s->st23[0], s->st23[1]};     // one per stage
     for (const WinOp& o : plan)
     {
         const int c = o.chunk, slot = window_slot(o.step, c, nch, ns);
@@ -1417,28 +1437,32 @@ int mpcf_run_window(mpcf_solver* s, int nsteps, double cfl, double dt_max, void*
                 break;
             }
             case WOP_DT:
+                if (o.step > 0) CK(cudaStreamWaitEvent(s->stream, s->ev_st[nch - 1], 0));   // the last stage 3
                 if ((rc = enqueue_dt(s, cfl, dt_max))) return rc;
                 break;
             case WOP_STAGE:
             {
-                const int k = o.stage, b = p ^ (k & 1);
-                if (k == 0) CK(cudaStreamWaitEvent(s->stream, s->ev_up[std::min(c + 1, nch - 1)], 0));
+                // stage k of chunk c follows stage k-1 (stage 1: the upload)
+                // of the chunks up to c+1, whose buffers its ghost planes
+                // copy; a stage of a chunk further up may run meanwhile
+                const int k = o.stage, b = p ^ (k & 1), hc = std::min(c + 1, nch - 1);
+                CK(cudaStreamWaitEvent(str[k], k == 0 ? s->ev_up[hc] : s->ev_k[k - 1][hc], 0));
                 const void* lo = c > 0 ? s->hdoms[window_slot(o.step, c - 1, nch, ns)].U[b] : nullptr;
                 const void* hi = c < nch - 1 ? s->hdoms[window_slot(o.step, c + 1, nch, ns)].U[b] : nullptr;
-                CK(launch_window_ghosts((int)esz, D.U[b], lo, hi, fs, plane, nsl, s->win_bc[0], s->win_bc[1], s->stream));
+                CK(launch_window_ghosts((int)esz, D.U[b], lo, hi, fs, plane, nsl, s->win_bc[0], s->win_bc[1], str[k]));
                 s->parity = b;
                 rc = enqueue_stage_tiles(s, kLSRK3[k][0], kLSRK3[k][1], false, k == 2, D.tile_begin,
-                                         D.tile_begin + D.tiles_x * D.tiles_y * D.tiles_z);
+                                         D.tile_begin + D.tiles_x * D.tiles_y * D.tiles_z, str[k], k);
                 s->parity = p0;
                 if (rc) return rc;
+                CK(cudaEventRecord(k == 2 ? s->ev_st[c] : s->ev_k[k][c], str[k]));
                 if (k == 2)
                 {
-                    CK(cudaEventRecord(s->ev_st[c], s->stream));
                     // the chunk below is no longer read (its top planes were
                     // this stage's lower ghost planes); the last chunk frees
                     // its own slot
-                    if (c > 0) CK(cudaEventRecord(s->ev_free_c[window_slot(o.step, c - 1, nch, ns)], s->stream));
-                    if (c == nch - 1) CK(cudaEventRecord(s->ev_free_c[slot], s->stream));
+                    if (c > 0) CK(cudaEventRecord(s->ev_free_c[window_slot(o.step, c - 1, nch, ns)], str[k]));
+                    if (c == nch - 1) CK(cudaEventRecord(s->ev_free_c[slot], str[k]));
                 }
                 break;
             }

@@ -145,7 +145,8 @@ int mpcf_run(mpcf_solver* s, int nsteps, double cfl, double dt_max, int use_grap
  * covered every chunk within 3 planes above, and each chunk of the new
  * state goes back on a second copy stream as soon as stage 3 has written
  * it; the next step's upload of a chunk follows its download (copies in
- * both directions overlap each other and the kernels).  The first step's dt
+ * both directions overlap each other and the kernels; each stage has its own
+ * stream, so stages of different chunks overlap too).  The first step's dt
  * comes from the sound speed reduced chunk by chunk as the chunks land;
  * later steps take the sound speed that stage 3 accumulated over the state
  * it wrote (the values the host receives and sends back), as mpcf_run does.
@@ -177,7 +178,7 @@ int mpcf_run_host(mpcf_solver* s, int nsteps, double cfl, double dt_max, void* c
  *   the stage before it covers chunk c+1; before each stage a kernel fills
  *   the slot's ghost planes from the neighbouring slots, or by the boundary
  *   condition at the domain's z faces), and its download, on two copy
- *   streams and the solver's stream.  The first step's dt comes from a pass
+ *   streams and one stream per stage.  The first step's dt comes from a pass
  *   that streams every chunk through the slots, from the last down, and
  *   reduces its sound speed (the first step reuses the chunks it leaves);
  *   later steps take what stage 3 accumulated.  Results are bit-identical
