@@ -313,8 +313,9 @@ __device__ __forceinline__ void weno_record(const typename Vec16<typename Pol::T
     constexpr bool kBranchFree = sizeof(T) == 8 && !Pol::kWeno3;
     bool ok = true;         // every quantity's weights are in that form's range
 #pragma unroll
-    for (int v = 0; v < 8 / kPer; ++v)
+    for (int w = 0; w < 8 / kPer; ++w)
     {
+        const int v = Pol::kFastWeno && kPer == 4 ? 1 - w : w;     // (the half record first: fewer spills)
         T y[5][kPer];
 #pragma unroll
         for (int j = 0; j < 5; ++j) unpack(sm[ad[j] + v * PP], y[j]);
@@ -566,9 +567,17 @@ stage_kernel(const StageArgs A)
             q[7] = (T)0;
             st8<T, L::kPP>(sm, MPCF_IN((int)(hc >> 12 & 0x3ffffu), L::kCurOff, L::kYOff), q);
         };
+        // the threads that convert halo cells, and the first two cells of
+        // each; in FP64 with bulk copies not the last two warps, which evaluate
+        // the faces around the tile in the same phase (fast form, 256^3: 10.8
+        // ms a step against 11.1; in FP32 29.6 against 29.1 at 512^3, and
+        // slower with ordinary loads)
+        constexpr int kHalo = 6 * kTX + 6 * TY, kHaloThreads = (TMA && sizeof(T) == 8 && TY >= 7 ? TY - 2 : TY) * kTX;
         int hlx, hly;
         halo_place(threadIdx.x, hlx, hly);
         const unsigned hc0 = halo_cell(hlx, hly, !inner);
+        halo_place(threadIdx.x + kHaloThreads, hlx, hly);
+        const unsigned hc1 = halo_cell(hlx, hly, !inner);
         // the own column's cell of a staged interior and the momenta its
         // boundary condition flips
         bool own_fx, own_fy;
@@ -753,41 +762,35 @@ stage_kernel(const StageArgs A)
                 T* smTw = reinterpret_cast<T*>(sm);
                 if constexpr (Pol::kFastWeno && sizeof(T) == 4)
                 {
-                    // 14 jobs, 7 quantities of the two rows and 7 of the two
-                    // columns; a row / column and its mirror image on the
-                    // other side are the two lanes of a pair.  The rows'
-                    // jobs go to the first warps, the columns' to the last.
-                    auto edge_pair = [&](const int b0, const int s0, const int d0, const int b1, const int s1, const int d1, const int q)
+                    // 12 jobs: the pairs (rho, u), (v, w), (p, G) and P alone
+                    // of each of the 3 of ghost_job (the stencil's pairs are
+                    // half a record: half the loads and bank conflicts of one
+                    // quantity on two sides)
+#pragma unroll 1
+                    for (int e = ty; e < 12; e += TY)
                     {
-                        const int off = (q & 3) + (q >> 2) * (L::kPP * 4);
-                        float a0[5], a1[5];
+                        int base, step, dst;
+                        if (!ghost_job<L, TY>(e >> 2, tx, base, step, dst)) continue;
+                        const int q = 2 * (e & 3), off = (q & 3) + (q >> 2) * (L::kPP * 4);
+                        int ad[5];
 #pragma unroll
-                        for (int i = 0; i < 5; ++i)
-                        {
-                            a0[i] = smT[MPCF_IN(b0 + (i - 2) * s0, L::kCurOff, L::kYOff) * 4 + off];
-                            a1[i] = smT[MPCF_IN(b1 + (i - 2) * s1, L::kCurOff, L::kYOff) * 4 + off];
-                        }
-                        float2 r, l;
+                        for (int i = 0; i < 5; ++i) ad[i] = MPCF_IN(base + (i - 2) * step, L::kCurOff, L::kYOff) * 4 + off;
+                        const int at = MPCF_IN(dst, L::kYOff, L::kPP) * 4 + off;
                         if (q < 6)
-                            weno_edges<false, false>(make_float2(a0[0], a1[0]), make_float2(a0[1], a1[1]), make_float2(a0[2], a1[2]),
-                                              make_float2(a0[3], a1[3]), make_float2(a0[4], a1[4]), r, l);
+                        {
+                            float2 y[5], r, l;
+#pragma unroll
+                            for (int i = 0; i < 5; ++i) y[i] = *reinterpret_cast<const float2*>(smT + ad[i]);
+                            weno_edges<false, false>(y[0], y[1], y[2], y[3], y[4], r, l);
+                            *reinterpret_cast<float2*>(smTw + at) = r;
+                        }
                         else
                         {
-                            weno_edges<false, false>(a0[0], a0[1], a0[2], a0[3], a0[4], r.x, l.x);
-                            weno_edges<false, false>(a1[0], a1[1], a1[2], a1[3], a1[4], r.y, l.y);
+                            float r, l;
+                            weno_edges<false, false>(smT[ad[0]], smT[ad[1]], smT[ad[2]], smT[ad[3]], smT[ad[4]], r, l);
+                            smTw[at] = r;
                         }
-                        smTw[MPCF_IN(d0, L::kYOff, L::kPP) * 4 + off] = r.x;
-                        smTw[MPCF_IN(d1, L::kYOff, L::kPP) * 4 + off] = r.y;
-                    };
-#pragma unroll 1
-                    for (int q = ty; q < 7; q += TY)
-                        edge_pair(L::kCurOff + 2 * L::kCurW + tx + 3, L::kCurW, L::kYOff + tx,
-                                  L::kCurOff + (TY + 3) * L::kCurW + tx + 3, -L::kCurW, L::kTopOff + tx, q);
-                    if (tx < TY)
-#pragma unroll 1
-                        for (int q = TY - 1 - ty; q < 7; q += TY)
-                            edge_pair(L::kCurOff + (tx + 3) * L::kCurW + 2, 1, L::kXgOff + tx,
-                                      L::kCurOff + (tx + 3) * L::kCurW + kTX + 3, -1, L::kXlOff + tx, q);
+                    }
                 }
                 else
                 {
@@ -946,7 +949,6 @@ stage_kernel(const StageArgs A)
                 // corners are never read); a tile reaching past the domain
                 // converts the whole staged box, its out-of-domain cells
                 // mapped to their sources
-                constexpr int kHalo = 6 * kTX + 6 * TY;
                 if (box)
                 {
                     for (int i = threadIdx.x; i < (TY + 6) * L::kCurW; i += stage_threads<TY>())
@@ -955,10 +957,11 @@ stage_kernel(const StageArgs A)
                         convert_halo(halo_cell(lx, ly, true), 0, k + 1);
                     }
                 }
-                else
+                else if (threadIdx.x < (kHaloThreads < kHalo ? kHaloThreads : kHalo))
                 {
-                    if (threadIdx.x < kHalo) convert_halo(hc0, threadIdx.x, k + 1);
-                    for (int i = threadIdx.x + stage_threads<TY>(); i < kHalo; i += stage_threads<TY>())
+                    convert_halo(hc0, threadIdx.x, k + 1);
+                    if (threadIdx.x + kHaloThreads < kHalo) convert_halo(hc1, threadIdx.x + kHaloThreads, k + 1);
+                    for (int i = threadIdx.x + 2 * kHaloThreads; i < kHalo; i += kHaloThreads)
                     {
                         int lx, ly;
                         halo_place(i, lx, ly);
