@@ -56,15 +56,17 @@
 // DRAM traffic per cell-stage: read U (7 T) + read R (7 T) + write R and
 // U_next (14 T) = 112 B in FP32.  Halo and ring re-reads hit L2.
 //
-// What bounds it: instruction issue and the latency of dependent FP32
-// operations at 16 warps per SM (the mixed form: 1728 thread-instructions per
-// cell-stage, 62 % of the issue slots, FMA pipe 45 % and special-function
-// unit 46 % busy, DRAM 16 %).  512^3, 32 x 8 tiles, mixed: 28.9 ms a step
-// against 35.0 for one slab pass with face slots of 28 planes, three barriers
-// and two-sided fluxes; the parts: two phases, faces in registers, quantities
-// in packed pairs, upwind fluxes 32.8; halo addresses once per tile 30.6; the
-// row uniform to the compiler 30.0; y and x faces as a pair and the register
-// and state by bulk copy 28.9.
+// What bounds it: the latency of dependent FP32 operations, with shared
+// memory's, at 16 warps per SM (the mixed form, 256^3: 1615 thread-
+// instructions per cell-stage in 60 % of the issue slots, FMA pipe 49 %,
+// special-function unit 49 % and DRAM 19 % busy; fewer uniform-pipe
+// instructions or reciprocals did not help, fewer bank conflicts did).  512^3,
+// 32 x 8 tiles, mixed: 27.8 ms a step against 35.0 for one slab pass with
+// face slots of 28 planes, three barriers and two-sided fluxes; the parts: two
+// phases, faces in registers, quantities in packed pairs, upwind fluxes 32.8;
+// halo addresses once per tile 30.6; the row uniform to the compiler 30.0; y
+// and x faces as a pair and the register and state by bulk copy 28.9; ghost
+// edges in half records 27.8.
 #pragma once
 
 #include "mpcf_math.cuh"

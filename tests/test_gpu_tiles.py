@@ -90,3 +90,53 @@ def test_fp64_weights_over_the_range_of_scales(mpcf, prec, scale):
     for q in range(7):
         assert np.isfinite(Ug[q]).all()
         assert rel_linf(Ug[q], U[q]) <= 1e-8, (q, rel_linf(Ug[q], U[q]))
+
+
+@pytest.mark.parametrize("persistent", [False, True])
+@pytest.mark.parametrize("dims", [[(36, 9, 7), (33, 8, 5)], [(36, 9, 7), (64, 8, 5)]])
+def test_ensemble_rows_with_and_without_bulk_copies(mpcf, dims, persistent):
+    """Bulk copies are used when every domain's rows are multiples of 16
+    bytes; one other domain sends the whole solver to the ordinary loads.
+    One step of every domain, bit for bit."""
+    want, U0 = [], []
+    for i, d in enumerate(dims):
+        U = cloud_state(d, nb=1 + i)
+        U0.append([a.copy() for a in U])
+        R = [np.zeros_like(a) for a in U]
+        dt, _ = O.step(d, (ABS,) * 6, U, R, cfl=0.3)
+        want.append((dt, U, R))
+    with mpcf.Solver(dims, precision="fp32_ref") as s:
+        s.set_tiling(8, 3, persistent, True)
+        for i, U in enumerate(U0):
+            s.set_state(U, dom=i)
+        dts = s.step(cfl=0.3)
+        for i, (dt, U, R) in enumerate(want):
+            Ug, Rg = s.get_state(dom=i)
+            assert dts[i] == dt
+            assert_bitwise(Ug, U, f"domain {i}")
+            assert_bitwise(Rg, R, f"register of domain {i}")
+
+
+@pytest.mark.parametrize("prec", ["fp32_ref", "mixed", "fp64_fast"])
+def test_overlapping_stage_streams_match_resident_run(mpcf, prec):
+    """Streamed and windowed runs put each stage on its own stream: chunks
+    thinner than the stencil's reach and whole-depth ones, persistent and not,
+    against the resident run, bit for bit."""
+    dims = (40, 24, 30)
+    dt = mpcf.dtype_of(mpcf.PRECISIONS[prec])
+    U0 = [np.asarray(a, dt) for a in cloud_state(dims, nb=2)]
+    with mpcf.Solver([dims], precision=prec) as s:
+        s.set_state(U0)
+        s.run(3, cfl=0.3)
+        want = s.get_state(with_reg=False)
+    for dz, nchunks, persistent in ((2, 15, False), (2, 15, True), (5, 3, True), (30, 8, False)):
+        with mpcf.Solver([dims], precision=prec) as s:
+            s.set_tiling(8, dz, persistent, True)
+            host = [a.copy() for a in U0]
+            s.run_host(host, 3, cfl=0.3, nchunks=nchunks)
+        assert_bitwise(host, want, f"streamed, dz {dz}, persistent {persistent}")
+    for nslices, nslots in ((3, 5), (5, 6), (10, 3)):
+        with mpcf.WindowSolver(dims, nslices, nslots=nslots, precision=prec) as w:
+            host = [a.copy() for a in U0]
+            w.run(host, 3, cfl=0.3)
+        assert_bitwise(host, want, f"windowed, {nslices} planes")
