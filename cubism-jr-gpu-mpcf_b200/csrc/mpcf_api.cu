@@ -82,6 +82,10 @@ const double kLSRK3[3][2] = {{0.0, 1.0/4.0}, {-17.0/32.0, 8.0/9.0}, {-32.0/27.0,
 
 } // namespace
 
+// The copy count's word in a solver's counters (the words below it are the
+// work counters of launches that may overlap).
+constexpr int kCopyCount = 3;
+
 struct mpcf_solver
 {
     int device = 0;
@@ -102,7 +106,7 @@ struct mpcf_solver
     double* dt = nullptr;           // ndom
     double* time = nullptr;         // ndom
     unsigned* err = nullptr;        // 1
-    unsigned* counter = nullptr;    // 1
+    unsigned* counter = nullptr;    // 4: work counters of lanes 0..2 and, last, the copy count (kCopyCount)
     double* tile_sums = nullptr;    // ntiles * 5
     double* chunk_sums = nullptr;   // nchunks * 5
     double* sums = nullptr;         // ndom * 5
@@ -455,6 +459,7 @@ StageArgs stage_args(mpcf_solver* s, double a, double b, bool sums)
     A.b = b;
     A.dtinvh = s->dtinvh;
     A.counter = s->counter;
+    A.copy_count = s->test_flags ? s->counter + kCopyCount : nullptr;
     A.err = s->err;
     A.tile_sums = sums ? s->tile_sums : nullptr;
     A.tmaps = s->tmaps;
@@ -464,8 +469,8 @@ StageArgs stage_args(mpcf_solver* s, double a, double b, bool sums)
 }
 
 // Enqueue the stage of tiles [tile_lo, tile_hi) on the solver's stream, or
-// on stream `st` with the work counter of `lane` (launches that may overlap
-// have different lanes), with the device dt/h; the parity is left as it is
+// on stream `st` with the work counter of `lane` (0..kCopyCount-1; launches
+// that may overlap have different lanes), with the device dt/h; the parity is left as it is
 // (the caller flips it once the whole stage is enqueued).
 int enqueue_stage_tiles(mpcf_solver* s, double a, double b, bool sums, bool sos, int tile_lo, int tile_hi,
                         cudaStream_t st = nullptr, int lane = 0)
@@ -473,7 +478,7 @@ int enqueue_stage_tiles(mpcf_solver* s, double a, double b, bool sums, bool sos,
     if (!st) st = s->stream;
     StageArgs A = stage_args(s, a, b, sums);
     if (sos) A.sos_bits = s->sos_bits;
-    A.counter = s->counter + (lane ? lane + 1 : 0);     // (1 counts copies in failure-detection tests)
+    A.counter = s->counter + lane;
     A.tile0 = tile_lo;
     A.ntiles = tile_hi;
     int grid = tile_hi - tile_lo;
@@ -697,7 +702,7 @@ static int create_solver(mpcf_solver** out, int ndomains, const int* dims, const
     if ((rc = dev_alloc(s, (void**)&s->time, 8 * ndomains))) return bail(rc);
     if ((rc = dev_alloc(s, (void**)&s->sums, 8 * 5 * ndomains))) return bail(rc);
     if ((rc = dev_alloc(s, (void**)&s->err, 16))) return bail(rc);
-    if ((rc = dev_alloc(s, (void**)&s->counter, 16))) return bail(rc);
+    if ((rc = dev_alloc(s, (void**)&s->counter, sizeof(unsigned) * (kCopyCount + 1)))) return bail(rc);
     if ((rc = dev_alloc(s, &s->tmaps, (size_t)128 * 5 * ndomains))) return bail(rc);
     cudaMemsetAsync(s->sos_bits, 0, 8 * ndomains, s->stream);
     cudaMemsetAsync(s->dtinvh, 0, 8 * ndomains, s->stream);
@@ -705,7 +710,7 @@ static int create_solver(mpcf_solver** out, int ndomains, const int* dims, const
     cudaMemsetAsync(s->time, 0, 8 * ndomains, s->stream);
     cudaMemsetAsync(s->sums, 0, 8 * 5 * ndomains, s->stream);
     cudaMemsetAsync(s->err, 0, 16, s->stream);
-    cudaMemsetAsync(s->counter, 0, 16, s->stream);
+    cudaMemsetAsync(s->counter, 0, sizeof(unsigned) * (kCopyCount + 1), s->stream);
     if (cudaMallocHost(&s->host_stage, 8 * (size_t)ndomains * 8) != cudaSuccess)
     { cudaGetLastError(); return bail(fail(MPCF_ERR_NOMEM, "cudaMallocHost failed")); }
 
@@ -2294,8 +2299,8 @@ int mpcf_test_copy_count(mpcf_solver* s, unsigned* count, int clear)
 {
     if (!s || !count) return fail(MPCF_ERR_ARG, "null argument");
     DeviceGuard g(s->device);
-    CK(cudaMemcpyAsync(s->host_stage, s->counter + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, s->stream));
-    if (clear) CK(cudaMemsetAsync(s->counter + 1, 0, sizeof(unsigned), s->stream));
+    CK(cudaMemcpyAsync(s->host_stage, s->counter + kCopyCount, sizeof(unsigned), cudaMemcpyDeviceToHost, s->stream));
+    if (clear) CK(cudaMemsetAsync(s->counter + kCopyCount, 0, sizeof(unsigned), s->stream));
     CK(cudaStreamSynchronize(s->stream));
     *count = *(unsigned*)s->host_stage;
     return MPCF_OK;

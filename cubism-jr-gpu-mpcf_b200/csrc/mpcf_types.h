@@ -68,6 +68,7 @@ struct StageArgs
     double a, b;        // LSRK3 stage coefficients
     const void* dtinvh; // T[ndom], dt/h per domain
     unsigned* counter;  // persistent-launch work counter (zeroed before launch)
+    unsigned* copy_count; // counts the slabs' bulk copies in failure-detection tests, else null
     unsigned* err;      // device error word
     double* tile_sums;  // [ntiles][5] FP64 partial conservation sums, or null
     const void* tmaps;  // per domain 5 CUtensorMap (128 B each): [buffer 0, 1] x [halo box, interior box], register
@@ -81,8 +82,8 @@ struct StageArgs
 // with no copy in flight.  TEST_DROP_MID_COPY drops the chunk's first copy
 // after the prologue instead: the wait runs out one slab in, the CTA issues
 // no further copy and waits for the one still pending before it exits.
-// Persistent instances ignore both.  With any flag set, counter[1] counts the
-// bulk copies issued.
+// Persistent instances ignore both.  With any flag set, copy_count counts the
+// slabs' bulk copies (halo boxes and interiors).
 enum { TEST_DROP_LAST_COPY = 1u, TEST_DROP_MID_COPY = 2u };
 
 struct SosArgs

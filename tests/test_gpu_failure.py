@@ -90,3 +90,37 @@ def test_persistent_launches_ignore_the_test_flag(mpcf):
     with pytest.raises(mpcf.MpcfError):
         with mpcf.Solver([dims], precision="mixed") as s:
             s.set_test_flags(4)    # unknown flag
+
+
+@pytest.mark.parametrize("prec", ["mixed", "fp32_ref"])
+def test_copy_count_of_overlapping_persistent_launches(mpcf, prec):
+    """A test flag on a streamed and on a windowed run of persistent launches:
+    no copy is dropped, no tile is skipped (the result is that of the run
+    without the flag, bit for bit), and the count covers every launch of all
+    three stages: 2 d + 1 slab copies for a tile d planes deep (its d halo
+    boxes and d + 1 interiors)."""
+    dims, dz, steps = (64, 24, 30), 5, 2
+    U0 = [np.ascontiguousarray(a) for a in cloud_state(dims, nb=1)]
+    tiles = 2 * 3
+    got = []
+    for flag in (0, mpcf._lib.TEST_DROP_LAST_COPY):
+        with mpcf.Solver([dims], precision=prec) as s:
+            s.set_tiling(8, dz, persistent=True, tma=True)
+            s.set_test_flags(flag)
+            host = [a.copy() for a in U0]
+            s.run_host(host, steps, cfl=0.3, nchunks=3)
+            assert s.error_word() == 0
+            got.append(host)
+            assert s.test_copy_count() == (3 * steps * tiles * 6 * (2 * dz + 1) if flag else 0)
+    assert_bitwise(got[1], got[0], "streamed run with the flag")
+    got = []
+    for flag in (0, mpcf._lib.TEST_DROP_LAST_COPY):
+        with mpcf.WindowSolver(dims, 6, nslots=5, precision=prec) as w:
+            w.set_tiling(8, 3, persistent=True, tma=True)
+            w.set_test_flags(flag)
+            host = [a.copy() for a in U0]
+            w.run(host, steps, cfl=0.3)
+            assert w.error_word() == 0
+            got.append(host)
+            assert w.test_copy_count() == (3 * steps * tiles * 10 * (2 * 3 + 1) if flag else 0)
+    assert_bitwise(got[1], got[0], "windowed run with the flag")
