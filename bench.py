@@ -661,10 +661,6 @@ def e2e_measure(mpcf, cfg, K, W, cfl, dist, precision="mixed", tiling=None, nchu
     import torch
     s = make_solver(mpcf, cfg, precision)
     L = mpcf.lib()
-    if tiling is not None:
-        ty, _, persist, tma = tiling
-        nz = cfg["dims"][0][2]
-        s.set_tiling(ty, max(1, nz // nchunks), persist, tma)
     dtype = torch.float64 if precision in ("fp64", "fp64_fast") else torch.float32
     esz = 8 if precision in ("fp64", "fp64_fast") else 4
     ncell = sum(d[0] * d[1] * d[2] for d in cfg["dims"])
@@ -695,8 +691,8 @@ def e2e_measure(mpcf, cfg, K, W, cfl, dist, precision="mixed", tiling=None, nchu
         s.run_host(host, W, cfl=cfl, nchunks=nchunks)
         sec = timed(lambda k: s.run_host(host, k, cfl=cfl, nchunks=nchunks), K)
         out["value"], _ = rp.throughput(dist, ncell, 3.0 * K, sec * 1e3, device="cuda" if dist is not None else None)
-        out["path"] = (f"mpcf_run_host: state in pinned host memory read and written every step, {nchunks} z-chunks, "
-                       f"tiling {list(s.tiling())}, host wall clock over {K} steps")
+        out["path"] = (f"mpcf_run_host: state in pinned host memory read and written every step, {s.stream_plan(nchunks)[0]} z-chunks, "
+                       f"tiles {s.stream_plan(nchunks)[1]} planes deep, host wall clock over {K} steps")
         # the bound of a streamed step: its bytes each way at the measured
         # rate of concurrent host-to-device and device-to-host copies
         pk = pcie_peak()

@@ -123,6 +123,7 @@ struct mpcf_solver
 
     // launch configuration
     int ty = 7, dz = 64, persist = 0, tma = 0;
+    bool own_depth = true;          // dz is the solver's choice (not set by mpcf_set_tiling)
     bool tma_all = false;           // every domain qualifies for bulk copies
     int ntiles = 0;
     int sos_chunk = 32768, nchunks = 0;
@@ -374,17 +375,19 @@ int resident_ctas(const mpcf_solver* s, int ty, bool persist, bool tma)
 // (35 us per stage in the mixed form; 16 gives 70, 2 gives 40), 192^3 48 to
 // 64, 256^3 32 to 64.  Domains of different sizes (several per launch) fill
 // the slots like a list schedule: total work plus half a CTA's length.
-// `nd` leading domains share a launch.
-int best_depth(const mpcf_solver* s, int ty, int nd, int nb, double* cost_out = nullptr)
+// `nd` leading domains share a launch; `planes` > 0: a launch covers that many
+// planes of them.
+int best_depth(const mpcf_solver* s, int ty, int nd, int nb, int planes = 0)
 {
     const double start = 1.0, alone = s->pol == MPCF_PREC_FP32 || s->pol == MPCF_PREC_MIXED ? 0.66 : 0.78;
     const long long sms = s->num_sms, slots = sms * nb;
+    auto depth_of = [&](const DomDev& D) { return planes > 0 ? std::min(planes, D.nz) : D.nz; };
     int deepest = 0;
     bool even = true;
     for (int d = 0; d < nd; ++d)
     {
         const DomDev& D = s->hdoms[d];
-        deepest = std::max(deepest, D.nz);
+        deepest = std::max(deepest, depth_of(D));
         even = even && D.nx == s->hdoms[0].nx && D.ny == s->hdoms[0].ny && D.nz == s->hdoms[0].nz;
     }
     int best = deepest, last = 0;
@@ -399,9 +402,9 @@ int best_depth(const mpcf_solver* s, int ty, int nd, int nb, double* cost_out = 
         for (int d = 0; d < nd; ++d)
         {
             const DomDev& D = s->hdoms[d];
-            const long long txy = (long long)((D.nx + 31) / 32) * ((D.ny + ty - 1) / ty), cz = (D.nz + dz - 1) / dz;
+            const long long txy = (long long)((D.nx + 31) / 32) * ((D.ny + ty - 1) / ty), cz = (depth_of(D) + dz - 1) / dz;
             ctas += txy * cz;
-            work += (double)txy * (D.nz + start * cz);
+            work += (double)txy * (depth_of(D) + start * cz);
         }
         double cost;
         if (even)
@@ -414,7 +417,6 @@ int best_depth(const mpcf_solver* s, int ty, int nd, int nb, double* cost_out = 
         cost = std::max(cost, (nb > 1 && ctas <= sms ? alone : 1.0) * (dz + start));
         if (cost < best_cost * 0.995) { best_cost = cost; best = dz; }
     }
-    if (cost_out) *cost_out = best_cost;
     return best;
 }
 
@@ -432,6 +434,7 @@ void default_tiling(mpcf_solver* s, int nd)
     s->tma = 1;                       // dropped by apply_tiling when no domain qualifies
     const int nb = resident_ctas(s, s->ty, false, tma);
     s->dz = best_depth(s, s->ty, nd, nb);
+    s->own_depth = true;
     long long ctas = 0;
     for (int d = 0; d < nd; ++d)
     {
@@ -441,9 +444,37 @@ void default_tiling(mpcf_solver* s, int nd)
     s->persist = (s->pol == MPCF_PREC_FP32 || s->pol == MPCF_PREC_MIXED) && ctas > (long long)nb * s->num_sms;
 }
 
-int persistent_grid(mpcf_solver* s, int ty)
+// CTAs of a persistent launch over `tiles` tiles.
+int persistent_grid(const mpcf_solver* s, int tiles)
 {
-    return std::min(s->ntiles, resident_ctas(s, ty, true, s->tma != 0) * s->num_sms);
+    return std::min(tiles, resident_ctas(s, s->ty, true, s->tma != 0) * s->num_sms);
+}
+
+// Chunks and tile depth of a streamed run (mpcf_run_host).  A depth the caller
+// set is kept, one tile layer a chunk at least.  The solver's own depth is for
+// launches over the whole domain, so a streamed run takes another: `nchunks`
+// chunks of at least 4 MB and 3 planes each, and best_depth over one chunk.
+// Measured with 1 to 12 chunks (ms a step, 10-step runs; one chunk has no
+// overlap): 256^3 FP32 reference rounding 29.0 in 1, 16.6 in 4, 13.7 in 8;
+// 96^3 (25 MB) 1.66 in 1, 1.08 in 6, 1.15 in 8; below 4 MB a chunk the copies'
+// and launches' own cost shows: 64^3 mixed 0.43 in 1, 0.55 in 8, 64x8x8 0.10
+// and 0.36.  Chunks of fewer planes than the stencil reaches wait for two
+// others (400x400x12 mixed: 1.92 in chunks of 3 planes, 2.05 in 2).
+void stream_plan(const mpcf_solver* s, int nchunks, int* chunks, int* depth)
+{
+    const DomDev& D = s->hdoms[0];
+    int dz = s->dz, n = nchunks;
+    if (s->own_depth)
+    {
+        const double bytes = 7.0 * D.nx * D.ny * D.nz * s->esz;
+        n = std::max(1, std::min({nchunks, (int)std::min(bytes / 4e6, 1e9), D.nz / 3}));
+        const int planes = (D.nz + n - 1) / n;
+        const int d = best_depth(s, s->ty, 1, resident_ctas(s, s->ty, s->persist != 0, s->tma != 0), planes);
+        const int layers = (planes + d - 1) / d;     // per chunk, of equal depth
+        dz = (planes + layers - 1) / layers;
+    }
+    *depth = dz;
+    *chunks = std::min(n, (D.nz + dz - 1) / dz);
 }
 
 StageArgs stage_args(mpcf_solver* s, double a, double b, bool sums)
@@ -470,13 +501,16 @@ StageArgs stage_args(mpcf_solver* s, double a, double b, bool sums)
 
 // Enqueue the stage of tiles [tile_lo, tile_hi) on the solver's stream, or
 // on stream `st` with the work counter of `lane` (0..kCopyCount-1; launches
-// that may overlap have different lanes), with the device dt/h; the parity is left as it is
-// (the caller flips it once the whole stage is enqueued).
+// that may overlap have different lanes), with the device dt/h; the tiles are
+// `dz` deep (0: the solver's depth; another only where one domain is launched
+// without sums, since the tile tables hold the solver's).  The parity is left
+// as it is (the caller flips it once the whole stage is enqueued).
 int enqueue_stage_tiles(mpcf_solver* s, double a, double b, bool sums, bool sos, int tile_lo, int tile_hi,
-                        cudaStream_t st = nullptr, int lane = 0)
+                        cudaStream_t st = nullptr, int lane = 0, int dz = 0)
 {
     if (!st) st = s->stream;
     StageArgs A = stage_args(s, a, b, sums);
+    if (dz) A.dz = dz;
     if (sos) A.sos_bits = s->sos_bits;
     A.counter = s->counter + lane;
     A.tile0 = tile_lo;
@@ -484,7 +518,7 @@ int enqueue_stage_tiles(mpcf_solver* s, double a, double b, bool sums, bool sos,
     int grid = tile_hi - tile_lo;
     if (s->persist)
     {
-        grid = std::min(grid, persistent_grid(s, s->ty));
+        grid = persistent_grid(s, grid);
         CK(cudaMemsetAsync(A.counter, 0, sizeof(unsigned), st));
     }
     cudaError_t e = launch_stage(s, A, grid, st);
@@ -964,6 +998,17 @@ int mpcf_run(mpcf_solver* s, int nsteps, double cfl, double dt_max, int use_grap
     return MPCF_OK;
 }
 
+int mpcf_stream_plan(const mpcf_solver* s, int nchunks, int* chunks, int* depth)
+{
+    if (!s || !chunks || !depth) return fail(MPCF_ERR_ARG, "null argument");
+    if (s->win_nch) return window_only(s, "mpcf_stream_plan");
+    if (nchunks < 1) return fail(MPCF_ERR_ARG, "nchunks < 1");
+    if (s->ndom != 1) return fail(MPCF_ERR_ARG, "mpcf_stream_plan: one domain is streamed (the solver has %d)", s->ndom);
+    DeviceGuard g(s->device);
+    stream_plan(s, nchunks, chunks, depth);
+    return MPCF_OK;
+}
+
 int mpcf_run_host(mpcf_solver* s, int nsteps, double cfl, double dt_max, void* const* host7, int nchunks,
                   double* time_out)
 {
@@ -983,13 +1028,14 @@ int mpcf_run_host(mpcf_solver* s, int nsteps, double cfl, double dt_max, void* c
     const size_t esz = s->esz;
     // chunks of whole tile layers (tiles never straddle two chunks); the
     // tiles of layers l0..l1-1 are the contiguous range l0*txy .. l1*txy-1
-    const int layers = D.tiles_z, txy = D.tiles_x * D.tiles_y;
-    const int nch = std::min(nchunks, layers);
+    int nch, dz;
+    stream_plan(s, nchunks, &nch, &dz);
+    const int layers = (D.nz + dz - 1) / dz, txy = D.tiles_x * D.tiles_y;
     std::vector<int> lc(nch + 1), zc(nch + 1);
     for (int c = 0; c <= nch; ++c)
     {
         lc[c] = (int)((long long)layers * c / nch);
-        zc[c] = std::min(D.nz, lc[c] * s->dz);
+        zc[c] = (int)std::min((long long)D.nz, (long long)lc[c] * dz);
     }
     // streams and events, made once
     int rc;
@@ -1077,7 +1123,7 @@ int mpcf_run_host(mpcf_solver* s, int nsteps, double cfl, double dt_max, void* c
             const int c = d[k]++;
             CK(cudaStreamWaitEvent(str[k], k == 0 ? s->ev_up[hi[c]] : s->ev_k[k - 1][hi[c]], 0));
             s->parity = p ^ (k & 1);
-            rc = enqueue_stage_tiles(s, kLSRK3[k][0], kLSRK3[k][1], false, k == 2, lc[c] * txy, lc[c + 1] * txy, str[k], k);
+            rc = enqueue_stage_tiles(s, kLSRK3[k][0], kLSRK3[k][1], false, k == 2, lc[c] * txy, lc[c + 1] * txy, str[k], k, dz);
             s->parity = p;
             if (rc) return rc;
             CK(cudaEventRecord(k == 2 ? s->ev_st[c] : s->ev_k[k][c], str[k]));
@@ -2278,6 +2324,7 @@ int mpcf_set_tiling(mpcf_solver* s, int ty, int dz, int flags)
     DeviceGuard g(s->device);
     s->ty = ty;
     s->dz = dz;
+    s->own_depth = false;
     s->persist = (flags & MPCF_TILE_PERSISTENT) != 0;
     s->tma = (flags & MPCF_TILE_TMA) != 0;
     return apply_tiling(s);
@@ -2341,7 +2388,7 @@ int mpcf_launch_shape(const mpcf_solver* s, long long* ntiles, long long* grid, 
 {
     if (!s) return fail(MPCF_ERR_ARG, "null solver");
     if (ntiles) *ntiles = s->ntiles;
-    if (grid) *grid = s->persist ? persistent_grid(const_cast<mpcf_solver*>(s), s->ty) : s->ntiles;
+    if (grid) *grid = s->persist ? persistent_grid(s, s->ntiles) : s->ntiles;
     if (threads) *threads = stage_block_threads(s->ty);
     return MPCF_OK;
 }
@@ -2485,6 +2532,7 @@ int mpcf_autotune(mpcf_solver* s, int reps, int* best3, double* best_ms)
     s->parity = saved_parity;
     s->ty = rc ? saved_ty : bty;
     s->dz = rc ? saved_dz : bdz;
+    if (!rc) s->own_depth = true;
     s->persist = rc ? saved_p : bp;
     s->tma = rc ? saved_m : bm;
     int rc2 = apply_tiling(s);

@@ -145,6 +145,12 @@ class Solver:
                                   int(nchunks), ctypes.byref(t)))
         return t.value
 
+    def stream_plan(self, nchunks=8):
+        """(chunks, tile depth) of run_host (mpcf_stream_plan)."""
+        n, dz = ctypes.c_int(), ctypes.c_int()
+        check(lib().mpcf_stream_plan(self._h, int(nchunks), ctypes.byref(n), ctypes.byref(dz)))
+        return n.value, dz.value
+
     # -- stream-ordered building blocks (nothing synchronises) -------------
     def stream_handle(self):
         """The solver's cudaStream_t as an integer (mpcf_stream)."""

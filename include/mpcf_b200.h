@@ -150,13 +150,17 @@ int mpcf_run(mpcf_solver* s, int nsteps, double cfl, double dt_max, int use_grap
  * comes from the sound speed reduced chunk by chunk as the chunks land;
  * later steps take the sound speed that stage 3 accumulated over the state
  * it wrote (the values the host receives and sends back), as mpcf_run does.
- * nchunks: requested chunks (at most the tile layers, nz/dz; one layer per
- * chunk with the tiling's dz).  The register stays on the device (stage 1
+ * nchunks: requested chunks.  After mpcf_set_tiling at most the tile layers,
+ * nz/dz; otherwise the tiles' depth is chosen for the chunks, and small
+ * domains are cut into fewer (at least 4 MB and 3 planes each).
+ * mpcf_stream_plan gives the chunks and the depth that a run will take.  The
+ * register stays on the device (stage 1
  * multiplies it by a = 0).  Results are bit-identical to mpcf_run on the
  * same state.  Single-domain solvers without halo faces; conservation
  * tracking is not applied.  time_out (optional): the time. */
 int mpcf_run_host(mpcf_solver* s, int nsteps, double cfl, double dt_max, void* const* host7, int nchunks,
                   double* time_out);
+int mpcf_stream_plan(const mpcf_solver* s, int nchunks, int* chunks, int* depth);
 /* Windowed runs: a domain held in host memory that may be larger than the
  * device's, streamed through a few device slots in z-chunks of nslices
  * planes (the reference's GPUlab with nslices < sizeZ: chunks of nslices

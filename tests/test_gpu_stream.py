@@ -90,3 +90,48 @@ def test_streamed_run_rejects_what_it_cannot_stream(mpcf):
             s.run_host([np.zeros(10, np.float32)] * 7, 1)
         with pytest.raises(mpcf.MpcfError):
             s.run_host([np.zeros(32 * 16 * 16, np.float32)] * 7, 1, nchunks=0)
+
+
+@pytest.mark.parametrize("prec,dims,chunks", [
+    ("mixed", (384, 384, 384), 8),         # whole depth is the best resident tiling here
+    ("fp64_fast", (192, 192, 192), 8),
+    ("fp32_ref", (192, 192, 192), 8),
+    ("mixed", (400, 400, 12), 4),          # chunks of 3 planes
+    ("fp32_ref", (96, 96, 96), 6),         # 25 MB: chunks of 4 MB
+    ("mixed", (64, 8, 8), 1),
+    ("fp64", (20, 17, 8), 1),
+])
+def test_default_solver_streams_in_chunks_of_its_size(mpcf, prec, dims, chunks):
+    """A new solver's depth is for launches over the whole domain; its
+    streamed runs choose chunks and tile depth for themselves, before and
+    after autotuning.  A depth that the caller set is kept."""
+    with mpcf.Solver([dims], precision=prec) as s:
+        n, dz = s.stream_plan(8)
+        assert n == chunks and n * dz <= dims[2] + n * n       # (equal layers, at most one plane over per chunk)
+        assert s.stream_plan(1)[0] == 1
+        if dims[0] * dims[1] * dims[2] < 1e6:
+            s.set_state(cloud_state(dims, nb=1, dtype=s.dtype))
+            s.autotune(reps=1)
+            assert s.stream_plan(8)[0] == chunks
+        s.set_tiling(8, 2, False, True)
+        assert s.stream_plan(8) == (min(8, (dims[2] + 1) // 2), 2)
+
+
+@pytest.mark.parametrize("prec,dims,nchunks", [("mixed", (257, 130, 95), 8), ("mixed", (256, 128, 100), 5),
+                                               ("fp32_ref", (260, 131, 61), 8), ("fp64_fast", (128, 70, 67), 8)])
+def test_default_streamed_run_equals_resident_run(mpcf, prec, dims, nchunks):
+    """Every default, ragged chunks and layers: bit for bit."""
+    U0 = [np.asarray(a, mpcf.dtype_of(mpcf.PRECISIONS[prec])) for a in cloud_state(dims, nb=3, seed=21)]
+    with mpcf.Solver([dims], precision=prec) as s:
+        s.set_state(U0)
+        s.run(2, cfl=0.3)
+        want = s.get_state(with_reg=False)
+    with mpcf.Solver([dims], precision=prec) as s:
+        host = [a.copy() for a in U0]
+        s.run_host(host, 2, cfl=0.3, nchunks=nchunks)
+        assert s.error_word() == 0
+        assert s.stream_plan(nchunks)[0] > 1
+        tiling = s.tiling()
+        s.run(1, cfl=0.3)
+        assert s.tiling() == tiling
+    assert_bitwise(host, want, f"default streamed run, {prec} {dims}")
