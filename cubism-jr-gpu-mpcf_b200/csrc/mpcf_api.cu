@@ -2493,8 +2493,12 @@ int mpcf_autotune(mpcf_solver* s, int reps, int* best3, double* best_ms)
         {
             if (!valid_ty(s, tys[i])) continue;
             // 8 rows are the fastest height; another is tried where its tiles
-            // cover a domain's rows with fewer rows in all
-            bool fewer = tys[i] == 8;
+            // cover a domain's rows with fewer rows in all, and the FP32
+            // reference form's 15 rows everywhere: half the CTAs can fit one
+            // round where those of 8 rows take two (us a stage, 15 against 8:
+            // 21x235x109 230 and 253, 128^3 544 and 563; 64^3 115 and 89; the
+            // other forms' 3 and 7 rows were never faster on 24 sizes)
+            bool fewer = tys[i] == 8 || tys[i] == 15;
             for (auto& D : s->hdoms) fewer = fewer || (D.ny + tys[i] - 1) / tys[i] * tys[i] < (D.ny + 7) / 8 * 8;
             if (!fewer) continue;
             for (int dz : dz_candidates(s, tys[i], maxn, can_tma))
