@@ -114,6 +114,11 @@ struct mpcf_solver
     int bubbles_cap = 0;
     void* host_stage = nullptr;     // pinned host scratch (ndom doubles/elems)
 
+    // ensembles with bulk-copy and other domains: the stream and the events
+    // (fork, join) of the second of a stage's two launches
+    cudaStream_t side = nullptr;
+    cudaEvent_t ev_side[2] = {nullptr, nullptr};
+
     void* tmaps = nullptr;          // ndom * 5 CUtensorMap (128 B each)
 
     // linked z-slabs (lower, upper) and their device copy
@@ -124,7 +129,7 @@ struct mpcf_solver
     // launch configuration
     int ty = 7, dz = 64, persist = 0, tma = 0;
     bool own_depth = true;          // dz is the solver's choice (not set by mpcf_set_tiling)
-    bool tma_all = false;           // every domain qualifies for bulk copies
+    int tma_tiles = 0;              // tiles of domains staged by bulk copies (the first ones)
     int ntiles = 0;
     int sos_chunk = 32768, nchunks = 0;
     bool track_cons = false;
@@ -186,10 +191,8 @@ StageKernelInfo stage_info(const mpcf_solver* s, int ty, bool persist, bool sums
     }
 }
 
-cudaError_t launch_stage(const mpcf_solver* s, const StageArgs& A, int grid, cudaStream_t st)
+cudaError_t launch_stage(const mpcf_solver* s, bool tma, const StageArgs& A, int grid, cudaStream_t st)
 {
-    // the bulk-copy instance takes domains that all qualify
-    const bool tma = s->tma && s->tma_all;
     if (s->weno3)
         return s->pol == 0 ? launch_stage_ref_w3(s->ty, s->persist != 0, tma, A, grid, st)
                            : launch_stage_fp64_w3(s->ty, s->persist != 0, tma, A, grid, st);
@@ -290,6 +293,9 @@ int dev_alloc(mpcf_solver* s, void** p, size_t bytes)
 // descriptors.
 int apply_tiling(mpcf_solver* s)
 {
+    int rc;
+    if ((rc = encode_tensor_maps(s))) return rc;
+    if (s->tma && !any_tma_ok(s)) s->tma = 0;
     int t = 0, c = 0;
     for (auto& D : s->hdoms)
     {
@@ -300,12 +306,28 @@ int apply_tiling(mpcf_solver* s)
         D.tiles_x = (D.nx + 31) / 32;
         D.tiles_y = (D.ny + s->ty - 1) / s->ty;
         D.tiles_z = (D.nz + s->dz - 1) / s->dz;
-        D.tile_begin = t;
-        t += D.tiles_x * D.tiles_y * D.tiles_z;
+        D.ntiles = D.tiles_x * D.tiles_y * D.tiles_z;
         const long long N = (long long)D.nx * D.ny * D.nz;
         D.sos_chunk_begin = c;
         D.sos_chunks = (int)((N + s->sos_chunk - 1) / s->sos_chunk);
         c += D.sos_chunks;
+    }
+    // the tiles of domains that bulk copies stage, then the others': each
+    // part is one launch of its own kernel instance
+    for (const bool bulk : {true, false})
+    {
+        for (auto& D : s->hdoms)
+        {
+            if ((s->tma && D.tma_ok) != bulk) continue;
+            D.tile_begin = t;
+            t += D.ntiles;
+        }
+        if (bulk) s->tma_tiles = t;
+    }
+    if (s->tma_tiles > 0 && s->tma_tiles < t && !s->side)
+    {
+        for (cudaEvent_t& e : s->ev_side) if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        CK(cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking));
     }
     s->ntiles = t;
     s->nchunks = c;
@@ -315,14 +337,9 @@ int apply_tiling(mpcf_solver* s)
         s->allocs.erase(std::remove(s->allocs.begin(), s->allocs.end(), (void*)s->tile_sums), s->allocs.end());
         s->tile_sums = nullptr;
     }
-    int rc = dev_alloc(s, (void**)&s->tile_sums, sizeof(double) * 5 * (size_t)std::max(t, 1));
-    if (rc) return rc;
+    if ((rc = dev_alloc(s, (void**)&s->tile_sums, sizeof(double) * 5 * (size_t)std::max(t, 1)))) return rc;
     if (!s->chunk_sums)
         if ((rc = dev_alloc(s, (void**)&s->chunk_sums, sizeof(double) * 5 * (size_t)std::max(c, 1)))) return rc;
-    if ((rc = encode_tensor_maps(s))) return rc;
-    if (s->tma && !any_tma_ok(s)) s->tma = 0;
-    s->tma_all = true;
-    for (const auto& D : s->hdoms) s->tma_all = s->tma_all && D.tma_ok;
     CK(cudaMemcpyAsync(s->ddoms, s->hdoms.data(), sizeof(DomDev) * s->ndom, cudaMemcpyHostToDevice, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     destroy_graphs(s);
@@ -444,10 +461,10 @@ void default_tiling(mpcf_solver* s, int nd)
     s->persist = (s->pol == MPCF_PREC_FP32 || s->pol == MPCF_PREC_MIXED) && ctas > (long long)nb * s->num_sms;
 }
 
-// CTAs of a persistent launch over `tiles` tiles.
-int persistent_grid(const mpcf_solver* s, int tiles)
+// CTAs of a persistent launch over `tiles` tiles of one kind.
+int persistent_grid(const mpcf_solver* s, int tiles, bool tma)
 {
-    return std::min(tiles, resident_ctas(s, s->ty, true, s->tma != 0) * s->num_sms);
+    return std::min(tiles, resident_ctas(s, s->ty, true, tma) * s->num_sms);
 }
 
 // Chunks and tile depth of a streamed run (mpcf_run_host).  A depth the caller
@@ -512,17 +529,37 @@ int enqueue_stage_tiles(mpcf_solver* s, double a, double b, bool sums, bool sos,
     StageArgs A = stage_args(s, a, b, sums);
     if (dz) A.dz = dz;
     if (sos) A.sos_bits = s->sos_bits;
-    A.counter = s->counter + lane;
-    A.tile0 = tile_lo;
-    A.ntiles = tile_hi;
-    int grid = tile_hi - tile_lo;
-    if (s->persist)
+    auto part = [&](int lo, int hi, bool tma, cudaStream_t str, int counter) -> int
     {
-        grid = persistent_grid(s, grid);
-        CK(cudaMemsetAsync(A.counter, 0, sizeof(unsigned), st));
-    }
-    cudaError_t e = launch_stage(s, A, grid, st);
-    if (e != cudaSuccess) return fail(MPCF_ERR_CUDA, "stage launch failed: %s", cudaGetErrorString(e));
+        A.counter = s->counter + counter;
+        A.tile0 = lo;
+        A.ntiles = hi;
+        int grid = hi - lo;
+        if (s->persist)
+        {
+            grid = persistent_grid(s, grid, tma);
+            CK(cudaMemsetAsync(A.counter, 0, sizeof(unsigned), str));
+        }
+        cudaError_t e = launch_stage(s, tma, A, grid, str);
+        if (e != cudaSuccess) return fail(MPCF_ERR_CUDA, "stage launch failed: %s", cudaGetErrorString(e));
+        return MPCF_OK;
+    };
+    // (with another depth the tiles of a single domain are all of one kind)
+    const int mid = s->tma_tiles == s->ntiles ? tile_hi : s->tma_tiles == 0 ? tile_lo : std::min(std::max(s->tma_tiles, tile_lo), tile_hi);
+    if (mid == tile_hi) return part(tile_lo, tile_hi, true, st, lane);
+    if (mid == tile_lo) return part(tile_lo, tile_hi, false, st, lane);
+    // an ensemble of both kinds (one launch at a time: the next lane's counter
+    // is free): the smaller part on the side stream and first, so that the
+    // larger one fills the slots around it
+    const bool tma_first = mid - tile_lo < tile_hi - mid;
+    CK(cudaEventRecord(s->ev_side[0], st));
+    CK(cudaStreamWaitEvent(s->side, s->ev_side[0], 0));
+    int rc = tma_first ? part(tile_lo, mid, true, s->side, lane + 1) : part(mid, tile_hi, false, s->side, lane + 1);
+    if (rc) return rc;
+    rc = tma_first ? part(mid, tile_hi, false, st, lane) : part(tile_lo, mid, true, st, lane);
+    if (rc) return rc;
+    CK(cudaEventRecord(s->ev_side[1], s->side));
+    CK(cudaStreamWaitEvent(st, s->ev_side[1], 0));
     return MPCF_OK;
 }
 
@@ -765,8 +802,9 @@ int mpcf_destroy(mpcf_solver* s)
     if (!s) return MPCF_OK;
     DeviceGuard g(s->device);
     if (s->stream) cudaStreamSynchronize(s->stream);
-    for (cudaStream_t c : {s->up, s->down, s->st23[0], s->st23[1]})
+    for (cudaStream_t c : {s->up, s->down, s->st23[0], s->st23[1], s->side})
         if (c) { cudaStreamSynchronize(c); cudaStreamDestroy(c); }
+    for (cudaEvent_t e : s->ev_side) if (e) cudaEventDestroy(e);
     for (auto* v : {&s->ev_up, &s->ev_st, &s->ev_down, &s->ev_free_c, &s->ev_free_d, &s->ev_k[0], &s->ev_k[1]})
         for (cudaEvent_t e : *v) cudaEventDestroy(e);
     if (s->ev_start) cudaEventDestroy(s->ev_start);
@@ -2388,7 +2426,12 @@ int mpcf_launch_shape(const mpcf_solver* s, long long* ntiles, long long* grid, 
 {
     if (!s) return fail(MPCF_ERR_ARG, "null solver");
     if (ntiles) *ntiles = s->ntiles;
-    if (grid) *grid = s->persist ? persistent_grid(s, s->ntiles) : s->ntiles;
+    if (grid)
+    {
+        const int other = s->ntiles - s->tma_tiles;
+        *grid = !s->persist ? s->ntiles : (s->tma_tiles ? persistent_grid(s, s->tma_tiles, true) : 0) +
+                                          (other ? persistent_grid(s, other, false) : 0);
+    }
     if (threads) *threads = stage_block_threads(s->ty);
     return MPCF_OK;
 }

@@ -37,8 +37,8 @@
 // ping-ponged (read U[parity], write U[parity^1]) so neighbouring tiles
 // always see the old state.
 //
-// Loads.  With TMA (solvers whose domains' rows are all multiples of 16
-// bytes), three staging buffers in shared memory are filled while a phase is
+// Loads.  With TMA (domains whose rows are multiples of 16 bytes; a launch
+// covers domains of one kind), three staging buffers in shared memory are filled while a phase is
 // worked on, by four bulk tensor copies per slab that one elected thread
 // issues: in phase I the halo of the next slab (a 40 x (TY+6) box, whose
 // out-of-domain cells are mapped to their mirror / clamp source inside the
@@ -466,7 +466,7 @@ stage_kernel(const StageArgs A)
     {
         // ---- decode tile -> domain, tile coordinates
         int d = 0;
-        while (d + 1 < A.ndom && A.doms[d + 1].tile_begin <= t) ++d;
+        while (d + 1 < A.ndom && (unsigned)(t - A.doms[d].tile_begin) >= (unsigned)A.doms[d].ntiles) ++d;
         const DomDev& DD = A.doms[d];
         // A slab with halo faces is seen as its extended domain, stored
         // ghost planes included (planes -zlo .. nz-1+zhi become 0 ..

@@ -39,7 +39,8 @@ struct DomDev
     int    nx, ny, nz;
     int    bc[6];
     int    tiles_x, tiles_y, tiles_z;
-    int    tile_begin;  // first global tile id of this domain
+    int    tile_begin;  // first global tile id of this domain (bulk-copy domains come first)
+    int    ntiles;      // tiles_x * tiles_y * tiles_z
     int    sos_chunk_begin;   // first global sound-speed chunk of this domain
     int    sos_chunks;
     int    tma_ok;      // 1: tensor maps of this domain are valid (rows of 16-byte multiples)

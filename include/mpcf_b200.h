@@ -65,7 +65,7 @@ typedef struct mpcf_solver mpcf_solver;
 
 /* stage-kernel tiling flags (mpcf_set_tiling / mpcf_get_tiling / mpcf_autotune) */
 #define MPCF_TILE_PERSISTENT 1  /* one CTA per resident slot pulling tiles from a work counter */
-#define MPCF_TILE_TMA        2  /* stage slabs with bulk tensor copies (all domains with nx*elem % 16 == 0) */
+#define MPCF_TILE_TMA        2  /* stage slabs with bulk tensor copies (domains with nx*elem % 16 == 0) */
 
 /* Bubble-cloud initial condition (liquid with gas bubbles; indicator
  * alpha = 0.5*(1 - tanh(phi/(width*h))), phi = distance to the nearest
@@ -450,9 +450,10 @@ int mpcf_get_time(mpcf_solver* s, int dom, double* t);
 /* ---- launch configuration ------------------------------------------------- *
  * tile = 32 x ty columns x dz slabs (ty 3, 7 or 8; 15 also for
  * MPCF_PREC_FP32_REF), one CTA of 32*ty threads per tile;
- * flags = MPCF_TILE_PERSISTENT | MPCF_TILE_TMA.  With MPCF_TILE_TMA, a solver
- * whose domains' rows are all multiples of 16 bytes stages their slabs with
- * bulk tensor copies (otherwise each thread copies its own cells).  A new solver starts with
+ * flags = MPCF_TILE_PERSISTENT | MPCF_TILE_TMA.  With MPCF_TILE_TMA, domains
+ * whose rows are multiples of 16 bytes stage their slabs with bulk tensor
+ * copies (in the others each thread loads its own cells; an ensemble of both
+ * kinds takes two launches a stage that run side by side).  A new solver starts with
  * 32 x 8 tiles and a depth chosen from its sizes.  mpcf_autotune times the
  * candidates on the solver's own state (which it leaves unchanged) and
  * keeps the fastest; best3 (optional) = {ty, dz, flags}, best_ms (optional)

@@ -95,9 +95,8 @@ def test_fp64_weights_over_the_range_of_scales(mpcf, prec, scale):
 @pytest.mark.parametrize("persistent", [False, True])
 @pytest.mark.parametrize("dims", [[(36, 9, 7), (33, 8, 5)], [(36, 9, 7), (64, 8, 5)]])
 def test_ensemble_rows_with_and_without_bulk_copies(mpcf, dims, persistent):
-    """Bulk copies are used when every domain's rows are multiples of 16
-    bytes; one other domain sends the whole solver to the ordinary loads.
-    One step of every domain, bit for bit."""
+    """Bulk copies are used by the domains whose rows are multiples of 16
+    bytes.  One step of every domain, bit for bit."""
     want, U0 = [], []
     for i, d in enumerate(dims):
         U = cloud_state(d, nb=1 + i)
@@ -153,3 +152,46 @@ def test_autotune_tries_fifteen_rows_in_the_reference_form(mpcf):
         s.set_tiling(15, 6, False, False)
         s.time_stages(2)
         assert best <= 1.05 * min(s.time_stages(2) for _ in range(3))
+
+
+@pytest.mark.parametrize("prec", ["fp32_ref", "mixed", "fp64_fast"])
+def test_bulk_copy_and_other_domains_of_one_ensemble(mpcf, prec):
+    """Domains with and without rows of 16-byte multiples, in turn: each kind
+    keeps its way to load (slab copies are counted for the first alone), and
+    every domain, its conservation sums and its dt equal those of a solver of
+    its own, bit for bit, launched plainly, persistently and as a graph."""
+    dims = [(33, 8, 5), (36, 9, 7), (41, 17, 6), (64, 8, 12), (32, 8, 9), (38, 25, 5)]
+    bulk = [d for d in dims if d[0] * (8 if prec.startswith("fp64") else 4) % 16 == 0]
+    assert 0 < len(bulk) < len(dims)
+    dt = mpcf.dtype_of(mpcf.PRECISIONS[prec])
+    U0 = [[np.asarray(a, dt) for a in cloud_state(d, nb=1 + i)] for i, d in enumerate(dims)]
+    want = []
+    for d, U in zip(dims, U0):
+        with mpcf.Solver([d], precision=prec) as s:
+            s.set_tiling(8, 3, False, False)
+            s.track_conservation(True)
+            s.set_state(U)
+            t = s.run(3, cfl=0.3)
+            want.append((t, s.get_state(), s.conserved_sums()))
+    copies = sum((-(-d[0] // 32)) * (-(-d[1] // 8)) * (2 * d[2] + -(-d[2] // 3)) for d in bulk)
+    for persistent in (False, True):
+        for graph in (False, True):
+            with mpcf.Solver(dims, precision=prec) as s:
+                s.set_tiling(8, 3, persistent, True)
+                assert s.tiling() == (8, 3, persistent, True)
+                s.track_conservation(True)
+                if persistent:
+                    s.set_test_flags(mpcf._lib.TEST_DROP_LAST_COPY)     # (counts; persistent launches drop none)
+                for i, U in enumerate(U0):
+                    s.set_state(U, dom=i)
+                t = s.run(3, cfl=0.3, graph=graph)
+                sums = s.conserved_sums()
+                assert s.error_word() == 0
+                for i, (tw, (Uw, Rw), sw) in enumerate(want):
+                    Ug, Rg = s.get_state(dom=i)
+                    assert t[i] == tw[0]
+                    assert np.array_equal(sums[i], sw[0])
+                    assert_bitwise(Ug, Uw, f"domain {i}, persistent {persistent}")
+                    assert_bitwise(Rg, Rw, f"register of domain {i}, persistent {persistent}")
+                if persistent:
+                    assert s.test_copy_count() == 9 * copies
