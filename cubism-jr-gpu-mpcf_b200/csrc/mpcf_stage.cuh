@@ -434,7 +434,7 @@ stage_kernel(const StageArgs A)
     {
         if (isA) { mbar_expect_tx(barA, (uint32_t)L::kABytes); tma_load_4d(smem_u32(stA), tmap, c0, c1, c2, 0, barA); pendA = true; parA = phA; }
         else     { mbar_expect_tx(barB, (uint32_t)L::kBBytes); tma_load_4d(smem_u32(stB), tmap + 128, c0, c1, c2, 0, barB); pendB = true; parB = phB; }
-        if (A.copy_count) atomicAdd(A.copy_count, 1u);
+        if (A.test_flags) atomicAdd(A.copy_count, 1u);
     };
     // bounded wait of this thread for the copy into buffer A, B or C (0, 1,
     // 2); thread 0 clears the copy's pending mark when it sees it complete
