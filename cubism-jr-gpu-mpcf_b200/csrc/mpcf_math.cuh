@@ -419,7 +419,14 @@ __device__ __forceinline__ void hllc_face(const FaceState<typename Pol::T>& S, c
     // side's transverse velocities still enter as 0*t: a NaN or an infinity
     // there reaches the fluxes as it does in the reference's sum (any other
     // non-finite quantity makes s*, and with it everything, NaN).
-    const T z1 = (T)0 * (s < 0 ? S.t1m : S.t1p), z2 = (T)0 * (s < 0 ? S.t2m : S.t2p);
+    // The signs of zeros follow: for s* > 0 the other side's flux has the sign
+    // of its quantity and is +0 where that is a zero of either sign, so a -0
+    // of this side stays -0 only beside a negative transverse velocity
+    // (z, +0 for t = -0) and becomes +0 in the others (the + z0 below, in the
+    // exactly rounding FP32 forms); for s* < 0 this side's zeros are +0.
+    const T z0 = (T)0;
+    const T o1 = s < 0 ? S.t1m : S.t1p, o2 = s < 0 ? S.t2m : S.t2p;
+    const T z1 = (T)0 * (sizeof(T) == 4 ? o1 + z0 : o1), z2 = (T)0 * (sizeof(T) == 4 ? o2 + z0 : o2);
 #pragma unroll 1
     for (int side = s < 0 ? 1 : 0; ; side = 1)
     {
@@ -461,6 +468,10 @@ __device__ __forceinline__ void hllc_face(const FaceState<typename Pol::T>& S, c
         {
 #pragma unroll
             for (int m = 0; m < kFaceOut; ++m) o[m] = f[m];
+            if constexpr (sizeof(T) == 4)
+            {
+                o[0] = o[0] + z0; o[5] = o[5] + z0; o[6] = o[6] + z0; o[7] = o[7] + z0;
+            }
             o[1] = o[1] + (dir == 0 ? (T)0 : z1);
             o[2] = o[2] + (dir == 1 ? (T)0 : (dir == 0 ? z1 : z2));
             o[3] = o[3] + (dir == 2 ? (T)0 : z2);

@@ -195,3 +195,31 @@ def test_bulk_copy_and_other_domains_of_one_ensemble(mpcf, prec):
                     assert_bitwise(Rg, Rw, f"register of domain {i}, persistent {persistent}")
                 if persistent:
                     assert s.test_copy_count() == 9 * copies
+
+
+def test_signs_of_zeros(mpcf):
+    """Gas (P = 0) in blocks of equal velocities with zeros of both signs and
+    pressure jumps that expand against slow inflow (u < 0 < s*): many fluxes
+    are zeros, whose sign the reference's blend of the two sides decides.
+    Every bit of state and register over three stages."""
+    dims = (40, 17, 12)
+    rng = np.random.default_rng(8)
+    block = np.stack(np.meshgrid(*[np.arange(n) // 2 for n in dims[::-1]], indexing="ij")).reshape(3, -1)
+    pick = lambda v: np.asarray(v)[rng.integers(0, len(v), (dims[2], dims[1], dims[0]))[tuple(block)]]   # noqa: E731
+    speeds = [0.0, -0.0, 1e-2, -1e-2, -1e-2]
+    rho, p = pick([1.0, 1.25, 2.0]), pick([1.0, 1.0, 8.0])
+    u, v, w = pick(speeds), pick(speeds), pick(speeds)
+    G = np.full_like(rho, 2.5)
+    U = [np.ascontiguousarray(a, np.float32) for a in (rho, rho * u, rho * v, rho * w, G * p + 0.5 * rho * (u * u + v * v + w * w), G, 0 * rho)]
+    R = [np.zeros_like(a) for a in U]
+    stages = ((0.0, 0.25, 0.05), (-17.0 / 32, 8.0 / 9, 0.05), (-32.0 / 27, 0.75, 0.05))
+    with mpcf.Solver([dims], precision="fp32_ref") as s:
+        s.set_state(U, R)
+        for st in stages:
+            s.stage(*st)
+        Ug, Rg = s.get_state()
+    for a, b, dtinvh in stages:
+        O.stage(dims, (ABS,) * 6, U, R, a, b, dtinvh)
+    for q in range(7):
+        for got, want, what in ((Ug[q], U[q], "state"), (Rg[q], R[q], "register")):
+            assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), (what, q, int((got.view(np.uint32) != want.view(np.uint32)).sum()))
