@@ -541,8 +541,9 @@ __device__ __forceinline__ void hllc_face_upwind(const FaceState<V>& S, FaceFlux
     const V sc = pick(left, dmin(splat<V>(0), sm), dmax(splat<V>(0), sp));
 
     const V chi = mul_(sub_(s, u), rcp_approx(sub_(s, ss)));
-    const V w   = pick(is_zero(sc), u, mul_(ss, chi));
     const V X   = mul_(sub_(ss, u), sc);
+    // (X = 0: S_ = 0, or s* = u and so chi = 1; a NaN s* is in X and in w)
+    const V w   = pick(is_zero(X), u, mul_(ss, chi));
     const V ke  = fma_(t2, t2, fma_(t1, t1, mul_(u, u)));
     const V E   = fma_(mul_(splat<V>(0.5), r), ke, fma_(G, p, P));
     o.r  = mul_(r, w);

@@ -223,3 +223,34 @@ def test_signs_of_zeros(mpcf):
     for q in range(7):
         for got, want, what in ((Ug[q], U[q], "state"), (Rg[q], R[q], "register")):
             assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), (what, q, int((got.view(np.uint32) != want.view(np.uint32)).sum()))
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("prec", ["fp32", "mixed", "fp64_fast"])
+def test_a_state_without_sound_speed_spreads_in_the_fast_forms(mpcf, prec, axis):
+    """Supersonic flow (Mach 8, along each axis and both ways) into a cell
+    whose pressure is below -pc: no real sound speed and no star speed, so
+    every flux of its faces is NaN, the supersonic neighbour's included.  All
+    seven fields lose the same cells as in the oracle, and the error word
+    says so."""
+    dims = (36, 12, 9)
+    shape = dims[::-1]
+    for way in (1.0, -1.0):
+        dt = np.float64 if prec == "fp64_fast" else np.float32
+        rho, p = np.ones(shape), np.ones(shape)
+        p[4, 6, 17] = -3.0
+        G, mom = np.full(shape, 2.5), [np.zeros(shape) for _ in range(3)]
+        mom[axis][:] = 10.0 * way
+        E = G * p + 0.5 * sum(m * m for m in mom)
+        U = [np.ascontiguousarray(a.reshape(-1), dt) for a in (rho, *mom, E, G, 0 * rho)]
+        R = [np.zeros_like(a) for a in U]
+        with mpcf.Solver([dims], precision=prec) as s:
+            s.set_state(U, R)
+            s.stage(0.0, 0.25, 0.01)
+            Ug, Rg = s.get_state()
+            assert s.error_word() & mpcf._lib.ERRBIT_NONPHYSICAL
+        O.stage(dims, (ABS,) * 6, U, R, 0.0, 0.25, 0.01)
+        for q in range(7):
+            assert np.isnan(U[q]).any()
+            assert np.array_equal(np.isnan(Ug[q]), np.isnan(U[q])), (q, int(np.isnan(Ug[q]).sum()), int(np.isnan(U[q]).sum()))
+            assert np.array_equal(np.isnan(Rg[q]), np.isnan(R[q])), q
