@@ -2625,6 +2625,20 @@ int mpcf_probe_fp32_peak(int device, double* tflops)
     return MPCF_OK;
 }
 
+int mpcf_probe_rcp64(int device, int rn, long long n, const double* x, double* y)
+{
+    if (!x || !y || n < 1) return fail(MPCF_ERR_ARG, "bad arguments");
+    DeviceGuard g(device);
+    double* d = nullptr;
+    CK(cudaMalloc(&d, sizeof(double) * 2 * (size_t)n));
+    cudaError_t e = cudaMemcpy(d, x, sizeof(double) * (size_t)n, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = launch_rcp_probe(d, d + n, n, rn, 0);
+    if (e == cudaSuccess) e = cudaMemcpy(y, d + n, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    if (e != cudaSuccess) return fail(MPCF_ERR_CUDA, "reciprocal probe failed: %s", cudaGetErrorString(e));
+    return MPCF_OK;
+}
+
 int mpcf_time_run(mpcf_solver* s, int nsteps, double cfl, double dt_max, double* ms)
 {
     Range nvtx("mpcf_time_run");

@@ -938,6 +938,20 @@ cudaError_t launch_fma_probe(int blocks, int iters, float* out, cudaStream_t st)
     return cudaGetLastError();
 }
 
+// The double-precision reciprocals of the stage kernel over an array: rn != 0
+// the reference form's (rcp_rn), else the fast form's (rcp_f64).
+__global__ void __launch_bounds__(256) rcp_probe_kernel(const double* x, double* y, long long n, int rn)
+{
+    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += 256LL * gridDim.x)
+        y[i] = rn ? rcp_rn(x[i]) : rcp_f64(x[i]);
+}
+
+cudaError_t launch_rcp_probe(const double* x, double* y, long long n, int rn, cudaStream_t st)
+{
+    rcp_probe_kernel<<<(unsigned)std::min((n + 255) / 256, 4096LL), 256, 0, st>>>(x, y, n, rn);
+    return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------------------
 // State update alone, U_next = b*R + U (the reference's _update,
 // GPUkernels.cu:1142-1179), for callers that run Convection and Update as

@@ -71,6 +71,7 @@ cudaError_t launch_window_ghosts(int esz, void* dst, const void* lo, const void*
                                  int nz, int bc_lo, int bc_hi, cudaStream_t st);
 cudaError_t launch_update(int is_double, const DomDev* doms, int ndom, int parity, double b, cudaStream_t st);
 cudaError_t launch_fma_probe(int blocks, int iters, float* out, cudaStream_t st);
+cudaError_t launch_rcp_probe(const double* x, double* y, long long n, int rn, cudaStream_t st);
 cudaError_t launch_sum_state(const DomDev* doms, int ndom, int parity, int nchunks, int chunk, int is_double,
                              double* chunk_sums, double* out, cudaStream_t st);
 

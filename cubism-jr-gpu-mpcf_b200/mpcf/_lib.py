@@ -146,6 +146,7 @@ SIGNATURES = {
     "mpcf_launch_shape": (_I, [_P, _c.POINTER(_c.c_longlong), _c.POINTER(_c.c_longlong), _PI]),
     "mpcf_time_stages": (_I, [_P, _I, _D, _PD]),
     "mpcf_probe_fp32_peak": (_I, [_I, _PD]),
+    "mpcf_probe_rcp64": (_I, [_I, _I, _c.c_longlong, _PD, _PD]),
     "mpcf_time_run": (_I, [_P, _I, _D, _D, _PD]),
     "mpcf_device_info": (_I, [_I, _c.c_char_p, _I, _c.POINTER(_c.c_longlong), _c.POINTER(_c.c_longlong), _PI]),
     "mpcf_device_synchronize": (_I, [_I]),

@@ -513,6 +513,10 @@ int mpcf_device_synchronize(int device);
 /* Measured FP32 CUDA-core throughput of the device (FMA chains), TFLOP/s:
  * the denominator of the stage kernel's compute roofline. */
 int mpcf_probe_fp32_peak(int device, double* tflops);
+/* y[i] = the stage kernel's reciprocal of x[i] in double precision (host
+ * arrays): rn != 0 the reference form's, else the fast form's.  For tests
+ * against IEEE division. */
+int mpcf_probe_rcp64(int device, int rn, long long n, const double* x, double* y);
 
 #ifdef __cplusplus
 }

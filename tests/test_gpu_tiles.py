@@ -65,11 +65,12 @@ def test_contact_at_rest_and_nan_velocity(mpcf):
 
 
 @pytest.mark.parametrize("prec", ["fp64", "fp64_fast"])
-@pytest.mark.parametrize("scale", [1.0, 1e16, 1e22, 1e60])
+@pytest.mark.parametrize("scale", [1.0, 1e16, 1e22, 1e60, 1e70, 1e74])
 def test_fp64_weights_over_the_range_of_scales(mpcf, prec, scale):
-    """Pressures from 1 to 1e60: above about 1e18 the fast form's shared
-    reciprocal leaves its range (1e22) and above 1e75 the reference form's
-    products would; both then take their general forms.  Random cells, so
+    """Pressures from 1 to 1e74: above about 1e18 the fast form's shared
+    reciprocal leaves its range (1e22), and above about 1e67 the sums of the
+    reference form's weights, of order 1 / (10 p^4), fall below 2^-900 (1e70);
+    both then take their general forms.  Random cells, so
     the indicators do not cancel; one stage against the FP64 oracle, whose
     1/6 of the extra terms is the reference's float literal, 5e-9 off: with
     dt/h divU of order 0.1 that moves G by less than 1e-8 (all else differs
@@ -254,3 +255,52 @@ def test_a_state_without_sound_speed_spreads_in_the_fast_forms(mpcf, prec, axis)
             assert np.isnan(U[q]).any()
             assert np.array_equal(np.isnan(Ug[q]), np.isnan(U[q])), (q, int(np.isnan(Ug[q]).sum()), int(np.isnan(U[q]).sum()))
             assert np.array_equal(np.isnan(Rg[q]), np.isnan(R[q])), q
+
+
+def reciprocals(mpcf, x, rn):
+    import ctypes
+    x = np.ascontiguousarray(x, np.float64)
+    y = np.empty_like(x)
+    pd = ctypes.POINTER(ctypes.c_double)
+    mpcf._lib.check(mpcf.lib().mpcf_probe_rcp64(0, int(rn), x.size, x.ctypes.data_as(pd), y.ctypes.data_as(pd)))
+    return y
+
+
+def reciprocal_arguments():
+    """What the stage kernel takes reciprocals of, and the edges of the
+    mantissa: powers of two and their neighbours, at exponents over +-900."""
+    rng = np.random.default_rng(3)
+    p = np.exp(rng.uniform(np.log(1e-6), np.log(1e38), (3, 1 << 20)))          # indicators + eps
+    p32 = p.astype(np.float32).astype(np.float64)
+    sums = []
+    for q in (1.0 / (10.0 * p * p), 1.0 / (10.0 * p32 * p32)):
+        sums += [q[0] + 6.0 * q[1] + 3.0 * q[2], q[2] + 6.0 * q[1] + 3.0 * q[0]]
+    scale = np.ldexp(1.0, rng.integers(-900, 900, 1 << 20).astype(np.int32))
+    k = rng.integers(0, 1 << 10, 1 << 20)
+    ulp = 2.0 ** -52
+    return np.concatenate([10.0 * p.ravel() * p.ravel(), 10.0 * p32.ravel() * p32.ravel(), *sums,
+                           scale * rng.uniform(1.0, 2.0, scale.size), scale * (1.0 + k * ulp),
+                           scale * (2.0 - (k + 2) * ulp)])
+
+
+def test_reference_form_reciprocal_rounds_like_division(mpcf):
+    """rcp_rn equals IEEE division on 1.3e7 arguments; for a mantissa of all
+    ones, where Markstein's theorem does not hold, it is at most one unit in
+    the last place off."""
+    x = reciprocal_arguments()
+    y = reciprocals(mpcf, x, True)
+    bad = y != 1.0 / x
+    assert not bad.any(), (int(bad.sum()), x[bad][:4].tolist())
+    ones = np.ldexp(2.0 - 2.0 ** -52, np.arange(-900, 900).astype(np.int32))
+    y, want = reciprocals(mpcf, ones, True), 1.0 / ones
+    assert (np.abs(y.view(np.int64) - want.view(np.int64)) <= 1).all()
+
+
+def test_fast_form_reciprocal_error(mpcf):
+    """rcp_f64: the approximation's error e (below 2^-19) becomes e^4 after
+    two Newton steps, below the rounding of the last, of relative size 2^-53,
+    plus the residual's own rounding times e^2: within one unit in the last
+    place of division."""
+    x = reciprocal_arguments()
+    y, want = reciprocals(mpcf, x, False), 1.0 / x
+    assert (np.abs(y.view(np.int64) - want.view(np.int64)) <= 1).all()
