@@ -2371,10 +2371,11 @@ int mpcf_set_tiling(mpcf_solver* s, int ty, int dz, int flags)
 int mpcf_set_test_flags(mpcf_solver* s, unsigned flags)
 {
     if (!s) return fail(MPCF_ERR_ARG, "null solver");
-    if (flags & ~(unsigned)(MPCF_TEST_DROP_LAST_COPY | MPCF_TEST_DROP_MID_COPY))
+    if (flags & ~(unsigned)(MPCF_TEST_DROP_LAST_COPY | MPCF_TEST_DROP_MID_COPY | MPCF_TEST_DROP_PLANE_COPY))
         return fail(MPCF_ERR_ARG, "unknown test flags 0x%x", flags);
     static_assert((unsigned)MPCF_TEST_DROP_LAST_COPY == (unsigned)TEST_DROP_LAST_COPY, "test flag");
     static_assert((unsigned)MPCF_TEST_DROP_MID_COPY == (unsigned)TEST_DROP_MID_COPY, "test flag");
+    static_assert((unsigned)MPCF_TEST_DROP_PLANE_COPY == (unsigned)TEST_DROP_PLANE_COPY, "test flag");
     s->test_flags = flags;
     destroy_graphs(s);   // captured launches carry the old flags
     return MPCF_OK;

@@ -834,10 +834,13 @@ stage_kernel(const StageArgs A)
                 {
                     fence_proxy_async();
                     mbar_expect_tx(barC, 2 * (uint32_t)L::kBBytes);
-                    tma_load_4d(smem_u32(stC), tmR, x0, y0, k - DD.zlo, 0, barC);
-                    tma_load_4d(smem_u32(stC + 7 * L::kRing), tm + 128, x0, y0, k, 0, barC);
-                    pendC = true;
-                    parC = phC;
+                    if (PERSIST || !((A.test_flags & TEST_DROP_PLANE_COPY) && k == z0))
+                    {
+                        tma_load_4d(smem_u32(stC), tmR, x0, y0, k - DD.zlo, 0, barC);
+                        tma_load_4d(smem_u32(stC + 7 * L::kRing), tm + 128, x0, y0, k, 0, barC);
+                        pendC = true;
+                        parC = phC;
+                    }
                 }
                 // ---- phase II: the y face below and the x face left of the
                 // own cell; the last two warps also the y faces above the

@@ -83,9 +83,11 @@ struct StageArgs
 // with no copy in flight.  TEST_DROP_MID_COPY drops the chunk's first copy
 // after the prologue instead: the wait runs out one slab in, the CTA issues
 // no further copy and waits for the one still pending before it exits.
-// Persistent instances ignore both.  With any flag set, copy_count counts the
+// TEST_DROP_PLANE_COPY drops the register and state of the chunk's first
+// plane: the wait before that plane is finalised runs out, with the next
+// slabs' copies pending.  Persistent instances ignore all three.  With any flag set, copy_count counts the
 // slabs' bulk copies (halo boxes and interiors).
-enum { TEST_DROP_LAST_COPY = 1u, TEST_DROP_MID_COPY = 2u };
+enum { TEST_DROP_LAST_COPY = 1u, TEST_DROP_MID_COPY = 2u, TEST_DROP_PLANE_COPY = 8u };
 
 struct SosArgs
 {

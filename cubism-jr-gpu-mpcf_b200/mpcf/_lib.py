@@ -32,6 +32,7 @@ ERRBIT_TMA_TIMEOUT = 4
 ERRBIT_TMA_INFLIGHT = 16
 TEST_DROP_LAST_COPY = 1
 TEST_DROP_MID_COPY = 2
+TEST_DROP_PLANE_COPY = 8
 TILE_PERSISTENT = 1
 TILE_TMA = 2
 

@@ -481,10 +481,14 @@ int mpcf_autotune(mpcf_solver* s, int reps, int* best3, double* best_ms);
  * the chunk's first copy after the prologue instead: the wait runs out one
  * slab in, the CTA issues no further copy, waits (bounded) for the copy it
  * issued with the dropped one, and exits with none in flight (a drain wait
- * that also ran out would set MPCF_ERRBIT_TMA_INFLIGHT).  Persistent launches
- * ignore both.  0 (the default) turns them off. */
+ * that also ran out would set MPCF_ERRBIT_TMA_INFLIGHT).
+ * MPCF_TEST_DROP_PLANE_COPY drops the copy of the register and state that the
+ * chunk's first plane is finalised from: that wait runs out with the next
+ * slabs' copies pending.  Persistent launches ignore all three.  0 (the
+ * default) turns them off. */
 #define MPCF_TEST_DROP_LAST_COPY 1u
 #define MPCF_TEST_DROP_MID_COPY  2u
+#define MPCF_TEST_DROP_PLANE_COPY 8u
 int mpcf_set_test_flags(mpcf_solver* s, unsigned flags);
 /* Failure-detection tests only: bulk copies of slabs (halo boxes and
  * interiors ahead of the march) the stage kernel issued while a test flag

@@ -124,3 +124,40 @@ def test_copy_count_of_overlapping_persistent_launches(mpcf, prec):
             got.append(host)
             assert w.test_copy_count() == (3 * steps * tiles * 10 * (2 * 3 + 1) if flag else 0)
     assert_bitwise(got[1], got[0], "windowed run with the flag")
+
+
+def test_the_wait_for_a_planes_register_and_state_runs_out(mpcf):
+    """The copy that a chunk's first plane is finalised from is dropped: the
+    wait before the finalisation runs out one slab later.  Six slab copies
+    were issued until then (the prologue's two and two slabs' pairs), none
+    after it; those pending are waited for (no MPCF_ERRBIT_TMA_INFLIGHT), and
+    the context stays usable.  Persistent launches ignore the flag."""
+    dims = (32, 8, 12)             # one 32x8 tile, two 6-slab chunks
+    U0 = cloud_state(dims, nb=1)
+    with mpcf.Solver([dims], precision="fp32_ref") as s:
+        s.set_tiling(8, 6, persistent=False, tma=True)
+        s.set_state(U0)
+        s.set_test_flags(mpcf._lib.TEST_DROP_PLANE_COPY)
+        s.test_copy_count(clear=True)
+        s.stage(0.0, 0.25, 0.05)
+        w = s.error_word(clear=True)
+        assert w & mpcf._lib.ERRBIT_TMA_TIMEOUT, hex(w)
+        assert not (w & mpcf._lib.ERRBIT_TMA_INFLIGHT), hex(w)
+        assert s.test_copy_count(clear=True) == 2 * 6
+        s.set_tiling(8, 6, persistent=True, tma=True)
+        s.set_state(U0)
+        s.stage(0.0, 0.25, 0.05)
+        assert s.error_word() == 0
+        s.set_test_flags(0)
+        s.set_tiling(8, 6, persistent=False, tma=True)
+        s.set_state(U0)
+        s.stage(0.0, 0.25, 0.05)
+        assert s.error_word() == 0
+        U, R = s.get_state()
+    with mpcf.Solver([dims], precision="fp32_ref") as f:
+        f.set_tiling(8, 6, persistent=False, tma=True)
+        f.set_state(U0)
+        f.stage(0.0, 0.25, 0.05)
+        Uf, Rf = f.get_state()
+    assert_bitwise(U, Uf, "state after the given-up stage")
+    assert_bitwise(R, Rf, "register after the given-up stage")
