@@ -169,9 +169,7 @@ struct mpcf_solver
 namespace {
 
 // Tile heights with stage-kernel instances: 3, 7 and 8 rows, and 15 for the
-// FP32 reference-rounding form.  Threads of one stage CTA: a warp per row.
-int stage_block_threads(int ty) { return 32 * ty; }
-
+// FP32 reference-rounding form.
 bool valid_ty(const mpcf_solver* s, int ty)
 {
     if (ty == 3 || ty == 7 || ty == 8) return true;
@@ -373,7 +371,7 @@ int resident_ctas(const mpcf_solver* s, int ty, bool persist, bool tma)
 {
     const StageKernelInfo I = stage_info(s, ty, persist, false, tma);
     int nb = 0;
-    if (!I.fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, I.fn, stage_block_threads(ty), I.smem) != cudaSuccess || nb < 1)
+    if (!I.fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, I.fn, I.threads, I.smem) != cudaSuccess || nb < 1)
     {
         cudaGetLastError();
         nb = 1;
@@ -2433,7 +2431,7 @@ int mpcf_launch_shape(const mpcf_solver* s, long long* ntiles, long long* grid, 
         *grid = !s->persist ? s->ntiles : (s->tma_tiles ? persistent_grid(s, s->tma_tiles, true) : 0) +
                                           (other ? persistent_grid(s, other, false) : 0);
     }
-    if (threads) *threads = stage_block_threads(s->ty);
+    if (threads) *threads = stage_info(s, s->ty, s->persist != 0, false, s->tma != 0).threads;
     return MPCF_OK;
 }
 
@@ -2536,13 +2534,14 @@ int mpcf_autotune(mpcf_solver* s, int reps, int* best3, double* best_ms)
         for (int i = 0; i < 4 && !rc; ++i)
         {
             if (!valid_ty(s, tys[i])) continue;
-            // 8 rows are the fastest height; another is tried where its tiles
-            // cover a domain's rows with fewer rows in all, and the FP32
-            // reference form's 15 rows everywhere: half the CTAs can fit one
-            // round where those of 8 rows take two (us a stage, 15 against 8:
-            // 21x235x109 230 and 253, 128^3 544 and 563; 64^3 115 and 89; the
-            // other forms' 3 and 7 rows were never faster on 24 sizes)
-            bool fewer = tys[i] == 8 || tys[i] == 15;
+            // 8 rows are the fastest height of the fast forms: another is
+            // tried where its tiles cover a domain's rows with fewer rows in
+            // all (none was faster elsewhere on 24 sizes).  The reference
+            // forms' 7 and 15 rows, with their helper warp, are tried
+            // everywhere (us a stage: FP64 251x383x13 602 with 7 against 635
+            // with 8, FP32 21x235x109 219 with 15 against 252, 128^3 512 and
+            // 564, but 64^3 109 and 90; 3 rows only won with fewer rows on 44)
+            bool fewer = tys[i] == 8 || (tys[i] >= 7 && (s->pol == MPCF_PREC_FP32_REF || s->pol == MPCF_PREC_FP64));
             for (auto& D : s->hdoms) fewer = fewer || (D.ny + tys[i] - 1) / tys[i] * tys[i] < (D.ny + 7) / 8 * 8;
             if (!fewer) continue;
             for (int dz : dz_candidates(s, tys[i], maxn, can_tma))

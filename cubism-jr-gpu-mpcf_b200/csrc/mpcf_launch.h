@@ -15,6 +15,7 @@ struct StageKernelInfo
 {
     const void* fn;     // kernel entry (for occupancy queries / attributes)
     size_t smem;        // dynamic shared memory per CTA
+    int threads;        // threads per CTA
 };
 
 // precision policy ids: 0 FP32 reference rounding, 1 fast FP32, 2 mixed, 3 FP64,

@@ -11,7 +11,8 @@
 // PCIe streaming (GPUlab.cpp:202-372,703-793); all state stays in HBM.
 //
 // Work decomposition.  A tile is 32 x TY columns in x-y and a z-chunk of
-// depth dz.  Warp w owns row w, one thread per column.  The CTA marches up
+// depth dz.  Warp w owns row w, one thread per column (in the reference forms
+// at heights 3, 7 and 15 one more warp takes the tile's rim).  The CTA marches up
 // the chunk one slab at a time, two phases and two barriers per slab k:
 //   I  the x/y flux differences of cell k-1 (its own faces in registers, the
 //      faces right of and above it from the neighbours); z: both edges of
@@ -267,6 +268,18 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* tmap, int 
                  :: "r"(dst), "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar) : "memory");
 }
 
+// Warps of one CTA: one per row and, in the reference-rounding forms at
+// heights 2^n - 1, a helper warp that owns no column: it reconstructs the ghost
+// edges around the tile and evaluates the faces above and right of it.
+// Without it 3 rows take 7 ghost edges per warp beside the 21 of its own
+// cells, 7 rows 3 and 15 rows 2, and with it the CTA has 2^n warps.  Without
+// and with it, us a stage: 3 rows, 240x9x377 FP64 623 and 469, FP32 359 and
+// 330; 7 rows, 112x62x128 FP32 304 and 292; 15 rows, 128^3 546 and 512.  (The
+// fast forms' reconstruction is too short a share to pay for a warp.)
+template <class Pol, int TY> __host__ __device__ constexpr bool stage_helper() { return !Pol::kFastWeno && ((TY + 1) & TY) == 0; }
+template <class Pol, int TY> __host__ __device__ constexpr int stage_warps() { return TY + (stage_helper<Pol, TY>() ? 1 : 0); }
+template <class Pol, int TY> __host__ __device__ constexpr int stage_threads() { return kTX * stage_warps<Pol, TY>(); }
+
 // Register budget: at least kMinWarpsPerSM resident warps per SM (128
 // registers per thread).  The slab's 21 reconstructions are independent, so
 // the compiler would otherwise trade occupancy for unbounded
@@ -275,14 +288,11 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* tmap, int 
 #ifndef MPCF_MIN_WARPS_PER_SM
 #define MPCF_MIN_WARPS_PER_SM 16
 #endif
-template <class T, int TY> struct MinBlocks
+template <class Pol, int TY> struct MinBlocks
 {
-    static constexpr int w = sizeof(T) == 8 ? MPCF_MIN_WARPS_PER_SM / 2 : MPCF_MIN_WARPS_PER_SM;
-    static constexpr int v = (w / TY) > 0 ? (w / TY) : 1;
+    static constexpr int w = sizeof(typename Pol::T) == 8 ? MPCF_MIN_WARPS_PER_SM / 2 : MPCF_MIN_WARPS_PER_SM;
+    static constexpr int v = (w / stage_warps<Pol, TY>()) > 0 ? (w / stage_warps<Pol, TY>()) : 1;
 };
-
-// Threads of one CTA: a warp per row.
-template <int TY> __host__ __device__ constexpr int stage_threads() { return kTX * TY; }
 
 // Record `i` (index of its vector in a plane) of 8 values, read / written.
 template <class T, int PP>
@@ -387,7 +397,7 @@ __device__ __forceinline__ bool ghost_job(const int g, const int tx, int& base, 
 }
 
 template <class Pol, int TY, bool PERSIST, bool SUMS, bool TMA>
-__global__ void __launch_bounds__(stage_threads<TY>(), MinBlocks<typename Pol::T, TY>::v)
+__global__ void __launch_bounds__(stage_threads<Pol, TY>(), MinBlocks<Pol, TY>::v)
 stage_kernel(const StageArgs A)
 {
     typedef typename Pol::T T;
@@ -396,6 +406,7 @@ stage_kernel(const StageArgs A)
     // from phase I to phase II in the ring slot of slab k-2, free by then
     constexpr bool kStashLy = !Pol::kFastWeno;
     constexpr bool kPairFaces = Pol::kFastWeno && sizeof(T) == 4;   // the y and x faces as one packed pair
+    constexpr bool kHelp = stage_helper<Pol, TY>();
     typedef typename Vec16<T>::V V;
     extern __shared__ __align__(16) unsigned char smem_dyn[];
     // 128-byte aligned base (bulk tensor copies need it for their targets)
@@ -412,6 +423,7 @@ stage_kernel(const StageArgs A)
     const int tx = threadIdx.x & (kTX - 1);
     // (the shuffle tells the compiler that the row is uniform over the warp)
     const int ty = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+    const bool column = !kHelp || ty < TY;     // the warp owns a row of columns
     const T a = (T)A.a;
     const T b = (T)A.b;
     const T factor6 = (T)1.0f / (T)6.0f;   // GPUkernels.cu:1103
@@ -495,7 +507,7 @@ stage_kernel(const StageArgs A)
         const int z0 = DD.zlo + bz * A.dz;
         const int z1 = min(z0 + A.dz, DD.zlo + DD.nz);
         const int gx = x0 + tx, gy = y0 + ty;
-        const bool valid = (gx < D.nx) && (gy < D.ny);
+        const bool valid = column && (gx < D.nx) && (gy < D.ny);
         const int own = ty * kTX + tx;     // own column inside a ring slot
         // the tile's columns are all inside the domain: its ring holds the
         // exact primitives of every cur interior cell
@@ -574,7 +586,7 @@ stage_kernel(const StageArgs A)
         // the faces around the tile in the same phase (fast form, 256^3: 10.8
         // ms a step against 11.1; in FP32 29.6 against 29.1 at 512^3, and
         // slower with ordinary loads)
-        constexpr int kHalo = 6 * kTX + 6 * TY, kHaloThreads = (TMA && sizeof(T) == 8 && TY >= 7 ? TY - 2 : TY) * kTX;
+        constexpr int kHalo = 6 * kTX + 6 * TY, kHaloThreads = kHelp ? stage_threads<Pol, TY>() : (TMA && sizeof(T) == 8 && TY >= 7 ? TY - 2 : TY) * kTX;
         int hlx, hly;
         halo_place(threadIdx.x, hlx, hly);
         const unsigned hc0 = halo_cell(hlx, hly, !inner);
@@ -596,13 +608,16 @@ stage_kernel(const StageArgs A)
         if (use_tma && threadIdx.x == 0 && !tma_late) issue_for(z0 - 1);
 
         // ---- prologue: slabs z0-3 .. z0+1 of the own column into the ring
-#pragma unroll
-        for (int j = 0; j < 5; ++j)
+        if (column)
         {
-            T q[8];
-            load_prim<Pol>(D, U, gx, gy, z0 - 3 + j, q, oob);
-            q[7] = (T)0;
-            st8<T, L::kPP>(sm, ring(j), q);
+#pragma unroll
+            for (int j = 0; j < 5; ++j)
+            {
+                T q[8];
+                load_prim<Pol>(D, U, gx, gy, z0 - 3 + j, q, oob);
+                q[7] = (T)0;
+                st8<T, L::kPP>(sm, ring(j), q);
+            }
         }
 
         // carried from slab to slab: the z face below, the upper z edge and
@@ -624,7 +639,7 @@ stage_kernel(const StageArgs A)
             // the staging buffers are free again (phase II of slab k-1 is
             // behind the barrier): copy while this slab is worked on
             if (use_tma) { if (threadIdx.x == 0 && !tma_late && xy) issue_for(k); }
-            else if (k > z0 && tx < 28) prefetch_l1(pf + (long long)D.nx * D.ny * k);
+            else if (column && k > z0 && tx < 28) prefetch_l1(pf + (long long)D.nx * D.ny * k);
 
             // ---- phase I
             const bool fin = (k > z0) && valid;
@@ -642,7 +657,7 @@ stage_kernel(const StageArgs A)
             T S[7], dU = 0;
 #pragma unroll
             for (int m = 0; m < 7; ++m) S[m] = 0;
-            if (k > z0)
+            if (column && k > z0)
             {
                 T Fr[8], Fa[8];
 #pragma unroll
@@ -661,13 +676,14 @@ stage_kernel(const StageArgs A)
             // finalisation: rhs = a*R - dtinvh*div(F) (with the G/P extra
             // terms), R <- rhs, U_next <- b*rhs + U
             T Rv[8], Lv[8];
+            if (column)
             {
                 int ad[5];
 #pragma unroll
                 for (int j = 0; j < 5; ++j) ad[j] = ring(r2 + j);
                 weno_record<Pol, L::kPP>(sm, ad, Rv, Lv);
             }
-            if (k >= z0)
+            if (column && k >= z0)
             {
                 T zf[8];
                 face_hllc<Pol>(Rz, Lv, 2, zf);
@@ -718,8 +734,11 @@ stage_kernel(const StageArgs A)
                 for (int m = 0; m < 8; ++m) zfp[m] = zf[m];
             }
             if (k == z1) break;
+            if (column)
+            {
 #pragma unroll
-            for (int m = 0; m < 8; ++m) Rz[m] = Rv[m];
+                for (int m = 0; m < 8; ++m) Rz[m] = Rv[m];
+            }
 
             T Ly[8], Rx[8], Lx[8];
 #pragma unroll
@@ -729,19 +748,34 @@ stage_kernel(const StageArgs A)
                 // y, then x edges of the own cell.  The fast forms unroll the
                 // two; the reference-rounding forms, whose reconstruction is
                 // five times the code, keep one copy.
-                const T szG = Lv[5] + Rv[5], szP = Lv[6] + Rv[6];
-                T syG = 0, syP = 0;
+                // (The helper warp's three ghost jobs go through that copy.)
+                T szG = 0, szP = 0, syG = 0, syP = 0;
+                if (column) { szG = Lv[5] + Rv[5]; szP = Lv[6] + Rv[6]; }
                 constexpr int kXYUnroll = Pol::kFastWeno ? 2 : 1;
+                const int nj = column ? 2 : 3;
 #pragma unroll kXYUnroll
-                for (int j = 0; j < 2; ++j)
+                for (int j = 0; j < nj; ++j)
                 {
-                    const int step = j ? 1 : L::kCurW;
-                    const int base = L::kCurOff + (ty + 3) * L::kCurW + tx + 3;
+                    int step = j ? 1 : L::kCurW;
+                    int base = L::kCurOff + (ty + 3) * L::kCurW + tx + 3;
+                    int dst = -1;
+                    bool lower = false;         // (a ghost job's) wanted edge: the left or lower one
+                    if (kHelp && !column)
+                    {
+                        base = L::kCurOff + 2 * L::kCurW + tx + 3;      // (the idle lanes')
+                        if (ghost_job<L, TY>(j, tx, base, step, dst)) { lower = step < 0; step = lower ? -step : step; }
+                    }
                     int ad[5];
 #pragma unroll
                     for (int i = 0; i < 5; ++i) ad[i] = MPCF_IN(base + (i - 2) * step, L::kCurOff, L::kYOff);
                     weno_record<Pol, L::kPP>(sm, ad, Rv, Lv);
-                    if (j == 0)
+                    if (kHelp && !column)
+                    {
+#pragma unroll
+                        for (int m = 0; m < 7; ++m) Rv[m] = lower ? Lv[m] : Rv[m];
+                        if (dst >= 0) st8<T, L::kPP>(sm, MPCF_IN(dst, L::kYOff, L::kPP), Rv);
+                    }
+                    else if (j == 0)
                     {
                         st8<T, L::kPP>(sm, L::kYOff + own + kTX, Rv);
                         if constexpr (kStashLy) st8<T, L::kPP>(sm, ring(r2), Lv);
@@ -794,7 +828,7 @@ stage_kernel(const StageArgs A)
                         }
                     }
                 }
-                else
+                else if constexpr (!kHelp)
                 {
                     // 21 jobs (3 of ghost_job x 7 quantities) in contiguous
                     // ranges over the warps
@@ -843,8 +877,8 @@ stage_kernel(const StageArgs A)
                     }
                 }
                 // ---- phase II: the y face below and the x face left of the
-                // own cell; the last two warps also the y faces above the
-                // tile and the x faces right of it
+                // own cell; the last two warps (the helper warp, where there
+                // is one) the y faces above the tile and the x faces right of it
                 if constexpr (kPairFaces)
                 {
                     T my[8], mx[8];
@@ -858,9 +892,9 @@ stage_kernel(const StageArgs A)
                 }
                 constexpr int kFaceUnroll = Pol::kFastWeno ? 3 : 1;
 #pragma unroll kFaceUnroll
-                for (int j = kPairFaces ? 2 : 0; j < 3; ++j)
+                for (int j = kPairFaces || !column ? 2 : 0; j < (kHelp ? (column ? 2 : 4) : 3); ++j)
                 {
-                    if (j == 2 && ty < TY - 2) break;
+                    if (!kHelp && j == 2 && ty < TY - 2) break;
                     T m[8], p[8], f[8];
                     int dir, dst = -1;
                     if (j == 0)
@@ -883,7 +917,7 @@ stage_kernel(const StageArgs A)
                         if (tx == 0) ld8<T, L::kPP>(sm, L::kXgOff + ty, m);
                         dir = 0;
                     }
-                    else if (ty == TY - 1)
+                    else if (kHelp ? j == 2 : ty == TY - 1)
                     {
                         dst = L::kYOff + TY * kTX + tx;
                         ld8<T, L::kPP>(sm, dst, m);
@@ -914,8 +948,9 @@ stage_kernel(const StageArgs A)
             }
 
             // slab k+3 of the own column
-            if (use_tma) { wait_copy(1); phB ^= 1; }
+            if (column)
             {
+                if (use_tma) { wait_copy(1); phB ^= 1; }
                 T q[8];
                 if (use_tma)
                 {
@@ -938,7 +973,7 @@ stage_kernel(const StageArgs A)
             if (k + 1 < z1)
             {
                 const bool box = use_tma && !full;
-                if (!box)
+                if (!box && column)
                 {
                     // interior from the ring
                     T q[8];
@@ -956,7 +991,7 @@ stage_kernel(const StageArgs A)
                 // mapped to their sources
                 if (box)
                 {
-                    for (int i = threadIdx.x; i < (TY + 6) * L::kCurW; i += stage_threads<TY>())
+                    for (int i = threadIdx.x; i < (TY + 6) * L::kCurW; i += stage_threads<Pol, TY>())
                     {
                         const int ly = i / L::kCurW - 3, lx = i % L::kCurW - 3;
                         convert_halo(halo_cell(lx, ly, true), 0, k + 1);
@@ -984,7 +1019,7 @@ stage_kernel(const StageArgs A)
         {
             const bool bad = __syncthreads_or(sbad);
             const T m = shfl_max(smax);
-            if (tx == 0) sos_w[ty] = m;
+            if (tx == 0 && column) sos_w[ty] = m;
             __syncthreads();
             if (threadIdx.x < 32)
             {
@@ -1003,7 +1038,7 @@ stage_kernel(const StageArgs A)
                 double v = cs[m];
 #pragma unroll
                 for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-                if (tx == 0) red[ty * 5 + m] = v;
+                if (tx == 0 && column) red[ty * 5 + m] = v;
             }
             __syncthreads();
             if (threadIdx.x < 5)

@@ -16,7 +16,7 @@ struct StageDispatch
     template <int TY, bool P, bool S, bool M>
     static cudaError_t go(const StageArgs& A, int grid, cudaStream_t st)
     {
-        stage_kernel<Pol, TY, P, S, M><<<grid, stage_threads<TY>(), stage_smem_bytes<Pol, TY, M>(), st>>>(A);
+        stage_kernel<Pol, TY, P, S, M><<<grid, stage_threads<Pol, TY>(), stage_smem_bytes<Pol, TY, M>(), st>>>(A);
         return cudaGetLastError();
     }
 
@@ -33,6 +33,7 @@ struct StageDispatch
     {
         StageKernelInfo I;
         I.smem = stage_smem_bytes<Pol, TY, M>();
+        I.threads = stage_threads<Pol, TY>();
         if (persist) I.fn = sums ? (const void*)stage_kernel<Pol, TY, true, true, M> : (const void*)stage_kernel<Pol, TY, true, false, M>;
         else         I.fn = sums ? (const void*)stage_kernel<Pol, TY, false, true, M> : (const void*)stage_kernel<Pol, TY, false, false, M>;
         return I;
@@ -64,8 +65,8 @@ struct StageDispatch
             case 15:
                 if (kWithTY15)
                     return tma ? info_ty<kWithTY15 ? 15 : 7, true>(persist, sums) : info_ty<kWithTY15 ? 15 : 7, false>(persist, sums);
-                { StageKernelInfo I = {nullptr, 0}; return I; }
-            default: { StageKernelInfo I = {nullptr, 0}; return I; }
+                { StageKernelInfo I = {nullptr, 0, 0}; return I; }
+            default: { StageKernelInfo I = {nullptr, 0, 0}; return I; }
         }
     }
 };

@@ -449,7 +449,8 @@ int mpcf_get_time(mpcf_solver* s, int dom, double* t);
 
 /* ---- launch configuration ------------------------------------------------- *
  * tile = 32 x ty columns x dz slabs (ty 3, 7 or 8; 15 also for
- * MPCF_PREC_FP32_REF), one CTA of 32*ty threads per tile;
+ * MPCF_PREC_FP32_REF), one CTA per tile, a warp per row (and, for ty 3, 7 and
+ * 15 in the reference-rounding forms, a helper warp for the tile's rim);
  * flags = MPCF_TILE_PERSISTENT | MPCF_TILE_TMA.  With MPCF_TILE_TMA, domains
  * whose rows are multiples of 16 bytes stage their slabs with bulk tensor
  * copies (in the others each thread loads its own cells; an ensemble of both

@@ -161,3 +161,29 @@ def test_the_wait_for_a_planes_register_and_state_runs_out(mpcf):
         Uf, Rf = f.get_state()
     assert_bitwise(U, Uf, "state after the given-up stage")
     assert_bitwise(R, Rf, "register after the given-up stage")
+
+
+def test_a_give_up_with_a_helper_warp(mpcf):
+    """The same at 7 rows in the reference form, whose helper warp waits for
+    the halo boxes alone: a dropped interior makes the columns' wait run out,
+    and the helper's own runs out at the next box, which is not issued."""
+    dims = (32, 7, 12)             # one 32x7 tile, two 6-slab chunks
+    U0 = cloud_state(dims, nb=1)
+    got = []
+    for flag in (mpcf._lib.TEST_DROP_MID_COPY, 0):
+        with mpcf.Solver([dims], precision="fp32_ref") as s:
+            s.set_tiling(7, 6, persistent=False, tma=True)
+            s.set_state(U0)
+            if flag:
+                s.set_test_flags(flag)
+                s.stage(0.0, 0.25, 0.05)
+                w = s.error_word(clear=True)
+                assert w & mpcf._lib.ERRBIT_TMA_TIMEOUT and not w & mpcf._lib.ERRBIT_TMA_INFLIGHT, hex(w)
+                assert s.test_copy_count() == 2 * 3
+                s.set_test_flags(0)
+                s.set_state(U0)
+            s.stage(0.0, 0.25, 0.05)
+            assert s.error_word() == 0
+            got.append(s.get_state())
+    for a, b, what in zip(*got, ("state", "register")):
+        assert_bitwise(a, b, what + " after the given-up stage")

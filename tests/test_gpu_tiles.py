@@ -304,3 +304,44 @@ def test_fast_form_reciprocal_error(mpcf):
     x = reciprocal_arguments()
     y, want = reciprocals(mpcf, x, False), 1.0 / x
     assert (np.abs(y.view(np.int64) - want.view(np.int64)) <= 1).all()
+
+
+@pytest.mark.parametrize("tma", [False, True])
+@pytest.mark.parametrize("prec,ty", [("fp32_ref", 3), ("fp32_ref", 7), ("fp32_ref", 15), ("fp64", 3), ("fp64", 7)])
+def test_heights_with_a_helper_warp(mpcf, prec, ty, tma):
+    """The reference forms' tiles of 2^n - 1 rows have a warp without columns:
+    state, register, dt and conservation sums over ragged tiles.  FP32: the
+    oracle's bits.  FP64: within 1e-12 of the 8-row tiles (whose instances
+    contract their expressions for themselves)."""
+    dims = (44, 2 * ty + 1, 9)
+    bc = (REF, ABS, ABS, REF, REF, ABS)
+    U0 = [np.asarray(a, mpcf.dtype_of(mpcf.PRECISIONS[prec])) for a in cloud_state(dims, nb=1)]
+    if prec == "fp32_ref":
+        U, R = [a.copy() for a in U0], [np.zeros_like(a) for a in U0]
+        dts = [O.step(dims, bc, U, R, cfl=0.3)[0] for _ in range(2)]
+    else:
+        with mpcf.Solver([dims], bc=[bc], precision=prec) as s:
+            s.set_tiling(8, 4, False, tma)
+            s.set_state(U0)
+            dts = [s.step(cfl=0.3)[0] for _ in range(2)]
+            U, R = s.get_state()
+    for persistent in (False, True):
+        with mpcf.Solver([dims], bc=[bc], precision=prec) as s:
+            s.set_tiling(ty, 4, persistent, tma)
+            assert s.launch_shape()[2] == 32 * (ty + 1)
+            s.track_conservation(True)
+            s.set_state(U0)
+            got = [s.step(cfl=0.3)[0] for _ in range(2)]
+            Ug, Rg = s.get_state()
+            sums = s.conserved_sums()[0]
+            assert s.error_word() == 0
+        for q in range(5):
+            assert abs(sums[q] - Ug[q].astype(np.float64).sum()) <= 1e-12 * np.abs(Ug[q].astype(np.float64)).sum()
+        if prec == "fp32_ref":
+            assert got == dts
+            assert_bitwise(Ug, U, f"state, {ty} rows, persistent {persistent}")
+            assert_bitwise(Rg, R, f"register, {ty} rows, persistent {persistent}")
+        else:
+            assert np.allclose(got, dts, rtol=1e-12, atol=0)
+            for q in range(7):
+                assert rel_linf(Ug[q], U[q]) <= 1e-12, (q, rel_linf(Ug[q], U[q]))
