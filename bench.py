@@ -42,7 +42,7 @@ METRIC = "cell-stage updates/s on 1 B200: mixed vs plain FP64 at stated L1 error
 UNIT = "cell-stage updates/s"
 BYTES_PER_CELL_STAGE = {"fp32_ref": 112, "fp32": 112, "mixed": 112, "fp64": 224, "fp64_fast": 224}
 # DRAM bytes per cell-stage of the mixed stage kernel measured by ncu
-# (dram__bytes_read.sum + dram__bytes_write.sum = 2.135 + 1.831 GB for one
+# (dram__bytes_read.sum + dram__bytes_write.sum = 2.210 + 1.836 GB for one
 # launch over the 512 x 512 x 128 lower quarter of the 512^3 cloud, 33.55 M
 # cells, 32 x 8 tiles over whole columns, persistent, bulk-copy staging: a
 # few-GB case of the bench's kernel and tiling).  The per-launch figure of the
@@ -52,7 +52,7 @@ DTYPE_OF = {"mixed": "f32+f64 (mixed)", "fp32": "f32", "fp32_ref": "f32 (referen
             "fp64_fast": "f64 (fast form)"}
 FORM_OF = {"mixed": "mixed form", "fp32": "fast FP32 form", "fp32_ref": "FP32 reference-rounding form",
            "fp64": "FP64 form", "fp64_fast": "fast FP64 form (factored algebra, refined reciprocals)"}
-MEASURED_DRAM_BYTES_PER_CELL_STAGE = {"mixed": (2.135219968e9 + 1.831107072e9) / (512 * 512 * 128)}
+MEASURED_DRAM_BYTES_PER_CELL_STAGE = {"mixed": (2.210188800e9 + 1.836040192e9) / (512 * 512 * 128)}
 
 
 # Algorithmic floating-point operations of one cell-stage, counted by
@@ -504,7 +504,8 @@ def main():
                                                              "fp64_fast": "Fast64"}[args.precision],
                          "ms_per_launch": st_ms,
                          "algorithmic_bytes_per_launch": bytes_launch, "peak_kind": peak_kind,
-                         "note": "the stage kernel is bound by the FP32 pipe, not HBM: see roofline_fp32"},
+                         "note": "the stage kernel is bound by the latency of dependent FP32 operations (FMA pipe 49 % busy), not HBM; "
+                                 "roofline_fp32 is the reference algorithm's operations, more than the kernel executes, over the FP32 peak"},
             "roofline_fp32": {"bound": "fp32", "achieved": ach_tf, "peak": fp32_peak.value, "unit": "TFLOP/s",
                               "frac": ach_tf / fp32_peak.value, "flops_per_cell_stage": FLOPS_PER_CELL_STAGE,
                               "peak_kind": "measured (mpcf_probe_fp32_peak, FMA chains)"},

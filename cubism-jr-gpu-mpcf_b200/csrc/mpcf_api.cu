@@ -387,8 +387,8 @@ int resident_ctas(const mpcf_solver* s, int ty, bool persist, bool tma)
 // (reference rounding) of the speed it has alone, and CTAs beyond the
 // resident ones wait for a slot.  So the best depth is the one whose CTAs
 // fill whole rounds of resident slots with the least start-up: 64^3 takes 4
-// (35 us per stage in the mixed form; 16 gives 70, 2 gives 40), 192^3 48 to
-// 64, 256^3 32 to 64.  Domains of different sizes (several per launch) fill
+// (35 us per stage in the mixed form; 16 gives 70, 2 gives 40), 192^3 96 in
+// FP32 and 192 in FP64, 256^3 32 or 64.  Domains of different sizes (several per launch) fill
 // the slots like a list schedule: total work plus half a CTA's length.
 // `nd` leading domains share a launch; `planes` > 0: a launch covers that many
 // planes of them.
